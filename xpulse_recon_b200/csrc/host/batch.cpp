@@ -32,6 +32,7 @@ struct StepPlan {
     int n_fwd = 0, n_err = 0, n_bwd = 0;
     uint32_t fwd_units = 0, bwd_units = 0;
     uint64_t max_n = 0;
+    bool multi = false;
 };
 
 // tuned schedules, per batch shape
@@ -102,6 +103,7 @@ int build_lists(xpr_batch *b, int splits, int layers, int column, cudaStream_t s
         P.fwd_units = it.fwd_units;
         P.bwd_units = it.bwd_units;
         P.max_n = it.max_n;
+        P.multi = it.multi;
         if (!it.fwd.empty()) P.fwd_off = append(it.fwd.data(), it.fwd.size() * sizeof(it.fwd[0]));
         if (!it.err.empty()) P.err_off = append(it.err.data(), it.err.size() * sizeof(it.err[0]));
         if (!it.bwd.empty()) P.bwd_off = append(it.bwd.data(), it.bwd.size() * sizeof(it.bwd[0]));
@@ -142,7 +144,7 @@ cudaError_t enqueue_forward(xpr_batch *b, uint32_t k, cudaStream_t s)
     const StepPlan &P = b->plan[k];
     if (!P.n_fwd) return cudaSuccess;
     return xpr::launch_forward_batched((const xpr::BatchFwdItem *)((char *)b->lists + P.fwd_off), P.n_fwd,
-                                       P.fwd_units, b->tickets, b->opts.arith, b->layers, b->grid_fwd, s);
+                                       P.fwd_units, b->tickets, b->opts.arith, b->layers, P.multi, b->grid_fwd, s);
 }
 
 cudaError_t enqueue_backward(xpr_batch *b, uint32_t k, cudaStream_t s)
@@ -151,7 +153,7 @@ cudaError_t enqueue_backward(xpr_batch *b, uint32_t k, cudaStream_t s)
     if (!P.n_bwd) return cudaSuccess;
     return xpr::launch_backward_batched((const xpr::BatchBwdItem *)((char *)b->lists + P.bwd_off), P.n_bwd,
                                         P.bwd_units, b->tickets + 2, b->opts.arith, b->opts.storage, b->column,
-                                        b->grid_bwd, s);
+                                        P.multi, b->grid_bwd, s);
 }
 
 cudaError_t enqueue_step(xpr_batch *b, uint32_t k, cudaStream_t s)

@@ -75,6 +75,7 @@ bool add_step_items(const PlannedProblem &pp, uint32_t k, int splits, int layers
     e.first = k == 0;
     out->max_n = out->max_n > npix ? out->max_n : npix;
     out->err.push_back(e);
+    out->multi |= p.modules > 1;
     BatchBwdItem w{};
     w.a = a;
     w.vol = p.vol;

@@ -42,6 +42,7 @@ struct StepItems {
     std::vector<BatchBwdItem> bwd;
     uint32_t fwd_units = 0, bwd_units = 0;
     uint64_t max_n = 0;
+    bool multi = false;            // some problem has several detector modules
     void clear()
     {
         fwd.clear();
@@ -49,6 +50,7 @@ struct StepItems {
         bwd.clear();
         fwd_units = bwd_units = 0;
         max_n = 0;
+        multi = false;
     }
 };
 

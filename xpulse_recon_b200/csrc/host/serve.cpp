@@ -471,14 +471,14 @@ void compute_loop(xpr_server *s)
             if (e == cudaSuccess) e = cudaEventRecord(s->tick_ev[h], s->comp);
             if (e == cudaSuccess && !items.fwd.empty())
                 e = xpr::launch_forward_batched((const xpr::BatchFwdItem *)db, (int)items.fwd.size(), items.fwd_units,
-                                                s->tickets, s->opts.arith, s->layers, s->grid_fwd, s->comp);
+                                                s->tickets, s->opts.arith, s->layers, items.multi, s->grid_fwd, s->comp);
             if (e == cudaSuccess)
                 e = xpr::launch_error_batched((const xpr::BatchErrItem *)(db + eo), (int)items.err.size(),
                                               s->opts.image_storage, s->opts.storage, items.max_n, *s->di, s->comp);
             if (e == cudaSuccess)
                 e = xpr::launch_backward_batched((const xpr::BatchBwdItem *)(db + bo), (int)items.bwd.size(),
                                                  items.bwd_units, s->tickets + 2, s->opts.arith, s->opts.storage, 16,
-                                                 s->grid_bwd, s->comp);
+                                                 items.multi, s->grid_bwd, s->comp);
         }
         ++tick;
         lk.lock();

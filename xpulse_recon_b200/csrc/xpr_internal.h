@@ -119,10 +119,11 @@ bool forward_layers_ok(int arith, int layers);
 int backward_brick(int axis, int cb);
 // kind 0: forward (cb = its brick layers), 1: backward (cb = its column length)
 int batched_ctas_per_sm(int kind, int arith, int dtype, int cb);
+// multi: some problem has several detector modules (the STRICT kernels for tilted projections)
 cudaError_t launch_forward_batched(const BatchFwdItem *items, int n_items, uint32_t total_units, uint32_t *ticket,
-                                   int arith, int layers, unsigned ctas, cudaStream_t s);
+                                   int arith, int layers, bool multi, unsigned ctas, cudaStream_t s);
 cudaError_t launch_backward_batched(const BatchBwdItem *items, int n_items, uint32_t total_units, uint32_t *ticket,
-                                    int arith, int dtype, int cb, unsigned ctas, cudaStream_t s);
+                                    int arith, int dtype, int cb, bool multi, unsigned ctas, cudaStream_t s);
 cudaError_t launch_error_batched(const BatchErrItem *items, int n_items, int image_dtype, int ratio_dtype,
                                  uint64_t max_n, const DeviceInfo &dev, cudaStream_t s);
 cudaError_t launch_fill_batched(const BatchFillItem *items, int n_items, uint64_t max_n, const DeviceInfo &dev,
