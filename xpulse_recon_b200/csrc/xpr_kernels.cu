@@ -1565,6 +1565,10 @@ __global__ void __launch_bounds__(NT, 4)
 // --------------------------------------------------------------------------------------
 // error, preprocessing, fill
 // --------------------------------------------------------------------------------------
+// The streaming kernels (error, preprocessing) move four elements per access when every buffer
+// allows it (16-byte alignment for 32-bit elements, 8 for 16-bit ones: `vec`), and element by
+// element otherwise and for the remainder; four elements per thread and step keep enough bytes in
+// flight for the memory's rate.
 template <int DT>
 __device__ __forceinline__ float load_any(const void *p, uint64_t i)
 {
@@ -1579,37 +1583,122 @@ __device__ __forceinline__ void store_any(void *p, uint64_t i, float v)
     else if (DT == kBF16) ((__nv_bfloat16 *)p)[i] = __float2bfloat16_rn(v);
     else ((__half *)p)[i] = __float2half_rn(v);
 }
+template <int DT>
+__device__ __forceinline__ void load4(const void *p, uint64_t q, float (&v)[4])  // elements 4 q .. 4 q + 3
+{
+    if (DT == kF32) {
+        const float4 a = ((const float4 *)p)[q];
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        return;
+    }
+    const uint2 a = ((const uint2 *)p)[q];
+    const uint32_t h[4] = {a.x & 0xffffu, a.x >> 16, a.y & 0xffffu, a.y >> 16};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        v[k] = DT == kBF16 ? __uint_as_float(h[k] << 16) : __half2float(__ushort_as_half((unsigned short)h[k]));
+}
+template <int DT>
+__device__ __forceinline__ void store4(void *p, uint64_t q, const float (&v)[4])
+{
+    if (DT == kF32) {
+        ((float4 *)p)[q] = make_float4(v[0], v[1], v[2], v[3]);
+        return;
+    }
+    uint32_t h[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        h[k] = DT == kBF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v[k])) : __half_as_ushort(__float2half_rn(v[k]));
+    ((uint2 *)p)[q] = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+}
 __device__ __forceinline__ float std_max(float a, float b) { return (a < b) ? b : a; }
+// whether a buffer of `dt` elements can be accessed four at a time
+__host__ __device__ __forceinline__ bool quads_ok(const void *p, int dt)
+{
+    return !(reinterpret_cast<uintptr_t>(p) & (dt == kF32 ? 15u : 7u));
+}
+
+// a / b (IEEE) for 2^-60 <= |b| <= 2^60: the exact division by b's reciprocal where neither the
+// dividend nor the quotient is near the ends of the range, the general one elsewhere.
+__device__ __forceinline__ float div_by(float a, float b, float y, float ylo)
+{
+    const float q = div_exact(a, -b, y, ylo);
+    return (fabsf(a) < 0x1p60f && fabsf(q) > 0x1p-60f) ? q : __fdiv_rn(a, b);
+}
+
+// p_logf of a positive normal number: its special cases aside, the same operations (the
+// quotient (m - 1) / (m + 1) with the divisor in [1.7, 2.5] by its reciprocal)
+__device__ __forceinline__ float p_logf_normal(float x)
+{
+    const uint32_t b = __float_as_uint(x);
+    int e = (int)(b >> 23) - 127;
+    float m = __uint_as_float((b & 0x7fffffu) | 0x3f800000u);
+    if (m > 0x1.6a09e6p+0f) { m = __fmul_rn(m, 0.5f); e += 1; }
+    const float d = __fadd_rn(m, 1.0f), y = rcp_screened(d);
+    const float s = div_exact(__fsub_rn(m, 1.0f), -d, y, __fmul_rn(__fmaf_rn(-d, y, 1.0f), y));
+    const float z = __fmul_rn(s, s);
+    float q = __fmaf_rn(z, 0x1.c71c72p-4f, 0x1.24924ap-3f);
+    q = __fmaf_rn(q, z, 0x1.99999ap-3f);
+    q = __fmaf_rn(q, z, 0x1.555556p-2f);
+    const float t = __fadd_rn(s, s);
+    const float lm = __fmaf_rn(t, __fmul_rn(z, q), t);
+    const float fe = (float)e;
+    return __fmaf_rn(fe, 0x1.62e4p-1f, __fmaf_rn(fe, 0x1.7f7d1cp-20f, lm));
+}
+__device__ __forceinline__ float p_logf_at_least_eps(float x)  // x >= kEps (infinity included) or NaN
+{
+    return x < __int_as_float(0x7f800000) ? p_logf_normal(x) : p_logf(x);
+}
+
+// FIXED_TO_FLOAT: the division by 2^22 is exact, a product
+__device__ __forceinline__ float fixed_to_float_mul(uint32_t x) { return __fmul_rn(__uint2float_rn(x), kEps); }
+
+// the log ratio of one pixel
+template <int MODE>
+__device__ __forceinline__ float ratio_of(float ref, float got, float w)
+{
+    if (MODE == XPR_ERROR_FIRST_1C) return p_logf_at_least_eps(std_max(ref, kEps));
+    // the divisor is in [2^-22, 2^10]
+    const float d = MODE == XPR_ERROR_STD ? fmaxf(got, kEps) : std_max(got, kEps);
+    const float y = rcp_screened(d);
+    const float q = div_by(ref, d, y, __fmul_rn(__fmaf_rn(-d, y, 1.0f), y));
+    return __fmul_rn(p_logf_at_least_eps(MODE == XPR_ERROR_STD ? fmaxf(q, kEps) : std_max(q, kEps)), w);
+}
+
+// Adds the warp's sum of squares to the residual.
+__device__ __forceinline__ void add_residual(double acc, double *residual)
+{
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0 && acc != 0.0) atomicAdd(residual, acc);
+}
 
 template <int MODE, int IDT, int RDT, bool ZERO, bool RESID>
 __global__ void k_error(const void *__restrict__ images, uint32_t *sum, void *ratio, uint64_t n, float w,
-                        double *residual)
+                        double *residual, int vec)
 {
     double acc = 0.0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float ref = load_any<IDT>(images, i);
-        const float got = fixed_to_float(sum[i]);
-        float r;
-        if (MODE == XPR_ERROR_STD) r = __fmul_rn(p_logf(fmaxf(__fdiv_rn(ref, fmaxf(got, kEps)), kEps)), w);
-        else if (MODE == XPR_ERROR_FIRST_1C) r = p_logf(std_max(ref, kEps));
-        else r = __fmul_rn(p_logf(std_max(__fdiv_rn(ref, std_max(got, kEps)), kEps)), w);
+    const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t quads = vec ? n / 4 : 0;
+    for (uint64_t q = t0; q < quads; q += step) {
+        float ref[4], r[4];
+        load4<IDT>(images, q, ref);
+        const uint4 s = ((const uint4 *)sum)[q];
+        const uint32_t got[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            r[k] = ratio_of<MODE>(ref[k], fixed_to_float_mul(got[k]), w);
+            if (RESID) acc += (double)r[k] * (double)r[k];
+        }
+        store4<RDT>(ratio, q, r);
+        if (ZERO) ((uint4 *)sum)[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    for (uint64_t i = 4 * quads + t0; i < n; i += step) {
+        const float r = ratio_of<MODE>(load_any<IDT>(images, i), fixed_to_float_mul(sum[i]), w);
         store_any<RDT>(ratio, i, r);
         if (ZERO) sum[i] = 0u;
         if (RESID) acc += (double)r * (double)r;
     }
-    if (RESID) {
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0 && acc != 0.0) atomicAdd(residual, acc);
-    }
+    if (RESID) add_residual(acc, residual);
 }
-
-// order-preserving float <-> int map for atomic min / max
-__device__ __forceinline__ int ford(float f)
-{
-    const int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float fordinv(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 __device__ __forceinline__ bool is_normal(float v)
 {
@@ -1617,84 +1706,130 @@ __device__ __forceinline__ bool is_normal(float v)
     return e != 0u && e != 0xffu;
 }
 
-__global__ void k_minmax(const float *__restrict__ x, uint64_t n, float *minmax)
+// Lowers *lo / raises *hi to a normal number, by the order of the bits: as an integer the order
+// of the floats that are not negative, as an unsigned one the reverse order of the negative ones.
+__device__ __forceinline__ void atomic_min_float(float *lo, float v)
+{
+    if (v >= 0.0f) atomicMin((int *)lo, __float_as_int(v));
+    else atomicMax((unsigned *)lo, __float_as_uint(v));
+}
+__device__ __forceinline__ void atomic_max_float(float *hi, float v)
+{
+    if (v >= 0.0f) atomicMax((int *)hi, __float_as_int(v));
+    else atomicMin((unsigned *)hi, __float_as_uint(v));
+}
+
+// minmax[0], minmax[1]: lowered / raised to the normal values of x
+__global__ void k_minmax(const float *__restrict__ x, uint64_t n, float *minmax, int vec)
 {
     float mn = FLT_MAX, mx = -FLT_MAX;
-    bool anyv = false;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float v = x[i];
-        if (is_normal(v)) {
-            mn = fminf(mn, v);
-            mx = fmaxf(mx, v);
-            anyv = true;
-        }
+    auto take = [&](float v) {
+        const bool ok = is_normal(v);
+        mn = ok ? fminf(mn, v) : mn;
+        mx = ok ? fmaxf(mx, v) : mx;
+    };
+    const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t quads = vec ? n / 4 : 0;
+#pragma unroll 4
+    for (uint64_t q = t0; q < quads; q += step) {
+        const float4 v = __ldg((const float4 *)x + q);
+        take(v.x);
+        take(v.y);
+        take(v.z);
+        take(v.w);
     }
+    for (uint64_t i = 4 * quads + t0; i < n; i += step) take(x[i]);
     for (int o = 16; o > 0; o >>= 1) {
         mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     }
-    anyv = __any_sync(0xffffffffu, anyv);
-    if ((threadIdx.x & 31) == 0 && anyv) {
-        atomicMin((int *)&minmax[0], ford(mn));
-        atomicMax((int *)&minmax[1], ford(mx));
+    __shared__ float s_mn[32], s_mx[32];
+    const int lane = threadIdx.x & 31, warps = blockDim.x / 32;
+    if (lane == 0) {
+        s_mn[threadIdx.x >> 5] = mn;
+        s_mx[threadIdx.x >> 5] = mx;
     }
-}
-
-// minmax[] holds ford()-encoded values while the reduction runs
-__global__ void k_minmax_encode(float *minmax, bool decode)
-{
+    __syncthreads();
     if (threadIdx.x == 0) {
-        if (!decode) {
-            const int a = ford(minmax[0]), b = ford(minmax[1]);
-            ((int *)minmax)[0] = a;
-            ((int *)minmax)[1] = b;
-        } else {
-            const float a = fordinv(((int *)minmax)[0]), b = fordinv(((int *)minmax)[1]);
-            minmax[0] = a;
-            minmax[1] = b;
+        for (int k = 1; k < warps; ++k) {
+            mn = fminf(mn, s_mn[k]);
+            mx = fmaxf(mx, s_mx[k]);
+        }
+        if (mn <= mx) {  // some value was normal
+            atomic_min_float(&minmax[0], mn);
+            atomic_max_float(&minmax[1], mx);
         }
     }
 }
 
-template <int ODT>
-__global__ void k_preprocess(const float *__restrict__ x, void *out, uint64_t n, int normalize,
-                             const float *__restrict__ minmax, int mlog)
-{
-    const float mn = normalize ? minmax[0] : 0.0f, mx = normalize ? minmax[1] : 0.0f;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        float v = x[i];
-        if (normalize) v = is_normal(v) ? __fdiv_rn(__fsub_rn(v, mn), __fsub_rn(mx, mn)) : __fdiv_rn(__fadd_rn(mx, mn), 2.0f);
+// What preprocessing does to one value (data_loader.hpp:48-101).
+struct Preprocess {
+    int normalize, mlog;
+    float mn, mx, range, y, ylo;
+    bool plain;  // the range's reciprocal can stand for it
+    __device__ __forceinline__ Preprocess(int normalize_, const float *minmax, int mlog_) : normalize(normalize_), mlog(mlog_)
+    {
+        mn = normalize ? minmax[0] : 0.0f;
+        mx = normalize ? minmax[1] : 0.0f;
+        range = __fsub_rn(mx, mn);
+        plain = fabsf(range) >= 0x1p-59f && fabsf(range) <= 0x1p59f;
+        y = rcp_screened(plain ? range : 1.0f);
+        ylo = __fmul_rn(__fmaf_rn(-range, y, 1.0f), y);
+    }
+    __device__ __forceinline__ float operator()(float v) const
+    {
+        if (normalize) {
+            if (!is_normal(v)) v = __fdiv_rn(__fadd_rn(mx, mn), 2.0f);
+            else if (plain) v = div_by(__fsub_rn(v, mn), range, y, ylo);
+            else v = __fdiv_rn(__fsub_rn(v, mn), range);
+        }
         if (mlog) {
             const float lo = 1.0f - kEps;
             float c = (lo < v) ? lo : v;          // std::min(v, 1 - eps)
             c = (c < kEps) ? kEps : c;            // std::max(., eps)
-            v = -p_logf(c);
+            v = -p_logf_at_least_eps(c);
         }
-        store_any<ODT>(out, i, v);
+        return v;
     }
+};
+
+template <int ODT>
+__global__ void k_preprocess(const float *__restrict__ x, void *out, uint64_t n, int normalize,
+                             const float *__restrict__ minmax, int mlog, int vec)
+{
+    const Preprocess f(normalize, minmax, mlog);
+    const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t quads = vec ? n / 4 : 0;
+    for (uint64_t q = t0; q < quads; q += step) {
+        float v[4];
+        load4<kF32>(x, q, v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = f(v[k]);
+        store4<ODT>(out, q, v);
+    }
+    for (uint64_t i = 4 * quads + t0; i < n; i += step) store_any<ODT>(out, i, f(x[i]));
 }
 
 // The preprocessing of k_preprocess applied to images [0, n_img) of W*H pixels in
 // acquisition order, each written to its subset-major slot (j mod S) * Pc + j / S
-// (dataset.hpp:133-140): one launch for a whole request's images.
+// (dataset.hpp:133-140): one launch for a whole request's images, a block row per image.
 template <int ODT>
 __global__ void k_preprocess_reorder(const float *__restrict__ x, void *out, uint64_t wh, uint32_t n_img, uint32_t S,
-                                     uint32_t Pc, int normalize, const float *__restrict__ minmax, int mlog)
+                                     uint32_t Pc, int normalize, const float *__restrict__ minmax, int mlog, int vec)
 {
-    const float mn = normalize ? minmax[0] : 0.0f, mx = normalize ? minmax[1] : 0.0f;
-    const uint64_t n = wh * n_img;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t j = i / wh, px = i - j * wh;
-        const uint64_t slot = (j % S) * Pc + j / S;
-        float v = x[i];
-        if (normalize) v = is_normal(v) ? __fdiv_rn(__fsub_rn(v, mn), __fsub_rn(mx, mn)) : __fdiv_rn(__fadd_rn(mx, mn), 2.0f);
-        if (mlog) {
-            const float lo = 1.0f - kEps;
-            float c = (lo < v) ? lo : v;          // std::min(v, 1 - eps)
-            c = (c < kEps) ? kEps : c;            // std::max(., eps)
-            v = -p_logf(c);
+    const Preprocess f(normalize, minmax, mlog);
+    const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    for (uint32_t j = blockIdx.y; j < n_img; j += gridDim.y) {
+        const uint64_t from = (uint64_t)j * wh, to = ((uint64_t)(j % S) * Pc + j / S) * wh;
+        const uint64_t quads = vec ? wh / 4 : 0;  // (vec: wh is a multiple of 4)
+        for (uint64_t q = t0; q < quads; q += step) {
+            float v[4];
+            load4<kF32>(x, from / 4 + q, v);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = f(v[k]);
+            store4<ODT>(out, to / 4 + q, v);
         }
-        store_any<ODT>(out, slot * wh + px, v);
+        for (uint64_t i = 4 * quads + t0; i < wh; i += step) store_any<ODT>(out, to + i, f(x[from + i]));
     }
 }
 
@@ -1808,18 +1943,28 @@ __global__ void k_error_batched(const BatchErrItem *__restrict__ items)
     const BatchErrItem I = items[blockIdx.y];
     double acc = 0.0;
     const bool resid = I.residual != nullptr;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < I.n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float ref = load_any<IDT>(I.images, i);
-        const float got = I.first ? 1.0f : fixed_to_float(I.sum[i]);
-        const float r = __fmul_rn(p_logf(fmaxf(__fdiv_rn(ref, fmaxf(got, kEps)), kEps)), I.weight);
+    const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t quads = quads_ok(I.images, IDT) && quads_ok(I.sum, kF32) && quads_ok(I.ratio, RDT) ? I.n / 4 : 0;
+    for (uint64_t q = t0; q < quads; q += step) {
+        float ref[4], r[4];
+        load4<IDT>(I.images, q, ref);
+        const uint4 s = ((const uint4 *)I.sum)[q];
+        const uint32_t got[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            r[k] = ratio_of<XPR_ERROR_STD>(ref[k], I.first ? 1.0f : fixed_to_float_mul(got[k]), I.weight);
+            if (resid) acc += (double)r[k] * (double)r[k];
+        }
+        store4<RDT>(I.ratio, q, r);
+        ((uint4 *)I.sum)[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    for (uint64_t i = 4 * quads + t0; i < I.n; i += step) {
+        const float r = ratio_of<XPR_ERROR_STD>(load_any<IDT>(I.images, i), I.first ? 1.0f : fixed_to_float_mul(I.sum[i]), I.weight);
         store_any<RDT>(I.ratio, i, r);
         I.sum[i] = 0u;
         if (resid) acc += (double)r * (double)r;
     }
-    if (resid) {
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((threadIdx.x & 31) == 0 && acc != 0.0) atomicAdd(I.residual, acc);
-    }
+    if (resid) add_residual(acc, I.residual);
 }
 
 __global__ void k_fill_batched(const BatchFillItem *__restrict__ items)
@@ -1832,9 +1977,9 @@ __global__ void k_fill_batched(const BatchFillItem *__restrict__ items)
 // ======================================================================================
 // launchers
 // ======================================================================================
-static inline unsigned stream_grid(uint64_t n, const DeviceInfo &dev)
+static inline unsigned stream_grid(uint64_t n, const DeviceInfo &dev, bool vec = false)
 {
-    const uint64_t want = (n + 255) / 256;
+    const uint64_t want = ((vec ? n / 4 : n) + 255) / 256;
     const uint64_t cap = (uint64_t)dev.sm_count * 8;
     return (unsigned)std::max<uint64_t>(1, std::min(want, cap));
 }
@@ -2041,52 +2186,52 @@ cudaError_t launch_backward(float *vol, const void *ratio, int dt, const xpr_pro
 
 template <int MODE, int IDT, int RDT>
 static void dispatch_error3(unsigned grid, cudaStream_t s, const void *img, uint32_t *sum, void *ratio, uint64_t n,
-                            float w, bool zero, double *res)
+                            float w, bool zero, double *res, int vec)
 {
     if (zero) {
-        if (res) k_error<MODE, IDT, RDT, true, true><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res);
-        else k_error<MODE, IDT, RDT, true, false><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res);
+        if (res) k_error<MODE, IDT, RDT, true, true><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res, vec);
+        else k_error<MODE, IDT, RDT, true, false><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res, vec);
     } else {
-        if (res) k_error<MODE, IDT, RDT, false, true><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res);
-        else k_error<MODE, IDT, RDT, false, false><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res);
+        if (res) k_error<MODE, IDT, RDT, false, true><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res, vec);
+        else k_error<MODE, IDT, RDT, false, false><<<grid, 256, 0, s>>>(img, sum, ratio, n, w, res, vec);
     }
 }
 
 template <int MODE, int IDT>
 static void dispatch_error2(int rdt, unsigned grid, cudaStream_t s, const void *img, uint32_t *sum, void *ratio,
-                            uint64_t n, float w, bool zero, double *res)
+                            uint64_t n, float w, bool zero, double *res, int vec)
 {
-    if (rdt == kBF16) dispatch_error3<MODE, IDT, kBF16>(grid, s, img, sum, ratio, n, w, zero, res);
-    else if (rdt == kF16) dispatch_error3<MODE, IDT, kF16>(grid, s, img, sum, ratio, n, w, zero, res);
-    else dispatch_error3<MODE, IDT, kF32>(grid, s, img, sum, ratio, n, w, zero, res);
+    if (rdt == kBF16) dispatch_error3<MODE, IDT, kBF16>(grid, s, img, sum, ratio, n, w, zero, res, vec);
+    else if (rdt == kF16) dispatch_error3<MODE, IDT, kF16>(grid, s, img, sum, ratio, n, w, zero, res, vec);
+    else dispatch_error3<MODE, IDT, kF32>(grid, s, img, sum, ratio, n, w, zero, res, vec);
 }
 
 template <int MODE>
 static void dispatch_error1(int idt, int rdt, unsigned grid, cudaStream_t s, const void *img, uint32_t *sum,
-                            void *ratio, uint64_t n, float w, bool zero, double *res)
+                            void *ratio, uint64_t n, float w, bool zero, double *res, int vec)
 {
-    if (idt == kBF16) dispatch_error2<MODE, kBF16>(rdt, grid, s, img, sum, ratio, n, w, zero, res);
-    else if (idt == kF16) dispatch_error2<MODE, kF16>(rdt, grid, s, img, sum, ratio, n, w, zero, res);
-    else dispatch_error2<MODE, kF32>(rdt, grid, s, img, sum, ratio, n, w, zero, res);
+    if (idt == kBF16) dispatch_error2<MODE, kBF16>(rdt, grid, s, img, sum, ratio, n, w, zero, res, vec);
+    else if (idt == kF16) dispatch_error2<MODE, kF16>(rdt, grid, s, img, sum, ratio, n, w, zero, res, vec);
+    else dispatch_error2<MODE, kF32>(rdt, grid, s, img, sum, ratio, n, w, zero, res, vec);
 }
 
 cudaError_t launch_error(const void *images, int idt, uint32_t *sum, void *ratio, int rdt, uint64_t n, float weight,
                          int mode, int zero_sum, double *residual, const DeviceInfo &dev, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    const unsigned grid = stream_grid(n, dev);
+    const int vec = quads_ok(images, idt) && quads_ok(sum, kF32) && quads_ok(ratio, rdt);
+    const unsigned grid = stream_grid(n, dev, vec);
     const bool zero = zero_sum && ((void *)sum != ratio);
-    if (mode == XPR_ERROR_FIRST_1C) dispatch_error1<XPR_ERROR_FIRST_1C>(idt, rdt, grid, s, images, sum, ratio, n, weight, zero, residual);
-    else if (mode == XPR_ERROR_1C) dispatch_error1<XPR_ERROR_1C>(idt, rdt, grid, s, images, sum, ratio, n, weight, zero, residual);
-    else dispatch_error1<XPR_ERROR_STD>(idt, rdt, grid, s, images, sum, ratio, n, weight, zero, residual);
+    if (mode == XPR_ERROR_FIRST_1C) dispatch_error1<XPR_ERROR_FIRST_1C>(idt, rdt, grid, s, images, sum, ratio, n, weight, zero, residual, vec);
+    else if (mode == XPR_ERROR_1C) dispatch_error1<XPR_ERROR_1C>(idt, rdt, grid, s, images, sum, ratio, n, weight, zero, residual, vec);
+    else dispatch_error1<XPR_ERROR_STD>(idt, rdt, grid, s, images, sum, ratio, n, weight, zero, residual, vec);
     return cudaGetLastError();
 }
 
 cudaError_t launch_minmax(const float *images, uint64_t n, float *minmax, const DeviceInfo &dev, cudaStream_t s)
 {
-    k_minmax_encode<<<1, 32, 0, s>>>(minmax, false);
-    if (n) k_minmax<<<stream_grid(n, dev), 256, 0, s>>>(images, n, minmax);
-    k_minmax_encode<<<1, 32, 0, s>>>(minmax, true);
+    const int vec = quads_ok(images, kF32);
+    if (n) k_minmax<<<stream_grid(n, dev, vec), 256, 0, s>>>(images, n, minmax, vec);
     return cudaGetLastError();
 }
 
@@ -2094,10 +2239,11 @@ cudaError_t launch_preprocess(const float *images, void *out, int odt, uint64_t 
                               int mlog, const DeviceInfo &dev, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    const unsigned grid = stream_grid(n, dev);
-    if (odt == kBF16) k_preprocess<kBF16><<<grid, 256, 0, s>>>(images, out, n, normalize, minmax, mlog);
-    else if (odt == kF16) k_preprocess<kF16><<<grid, 256, 0, s>>>(images, out, n, normalize, minmax, mlog);
-    else k_preprocess<kF32><<<grid, 256, 0, s>>>(images, out, n, normalize, minmax, mlog);
+    const int vec = quads_ok(images, kF32) && quads_ok(out, odt);
+    const unsigned grid = stream_grid(n, dev, vec);
+    if (odt == kBF16) k_preprocess<kBF16><<<grid, 256, 0, s>>>(images, out, n, normalize, minmax, mlog, vec);
+    else if (odt == kF16) k_preprocess<kF16><<<grid, 256, 0, s>>>(images, out, n, normalize, minmax, mlog, vec);
+    else k_preprocess<kF32><<<grid, 256, 0, s>>>(images, out, n, normalize, minmax, mlog, vec);
     return cudaGetLastError();
 }
 
@@ -2107,10 +2253,12 @@ cudaError_t launch_preprocess_reorder(const float *images, void *out, int odt, u
 {
     if (wh == 0 || n_img == 0) return cudaSuccess;
     if (S == 0 || Pc == 0 || n_img > S * Pc) return cudaErrorInvalidValue;
-    const unsigned grid = stream_grid(wh * n_img, dev);
-    if (odt == kBF16) k_preprocess_reorder<kBF16><<<grid, 256, 0, s>>>(images, out, wh, n_img, S, Pc, normalize, minmax, mlog);
-    else if (odt == kF16) k_preprocess_reorder<kF16><<<grid, 256, 0, s>>>(images, out, wh, n_img, S, Pc, normalize, minmax, mlog);
-    else k_preprocess_reorder<kF32><<<grid, 256, 0, s>>>(images, out, wh, n_img, S, Pc, normalize, minmax, mlog);
+    const int vec = quads_ok(images, kF32) && quads_ok(out, odt) && wh % 4 == 0;
+    const unsigned row = stream_grid(wh, dev, vec);  // blocks per image; enough images at once to fill the GPU
+    const dim3 grid(row, std::max(1u, std::min({n_img, 65535u, ((unsigned)dev.sm_count * 8 + row - 1) / row})));
+    if (odt == kBF16) k_preprocess_reorder<kBF16><<<grid, 256, 0, s>>>(images, out, wh, n_img, S, Pc, normalize, minmax, mlog, vec);
+    else if (odt == kF16) k_preprocess_reorder<kF16><<<grid, 256, 0, s>>>(images, out, wh, n_img, S, Pc, normalize, minmax, mlog, vec);
+    else k_preprocess_reorder<kF32><<<grid, 256, 0, s>>>(images, out, wh, n_img, S, Pc, normalize, minmax, mlog, vec);
     return cudaGetLastError();
 }
 
