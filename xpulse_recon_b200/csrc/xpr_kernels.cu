@@ -92,7 +92,8 @@ struct __align__(16) ProjMeta {
 // boundary and its rows are padded to a multiple of 4 words (the detector width must then
 // be a multiple of 4, which keeps the padded rows inside the image rows).
 // FILTER: the projections go by the filtered pixel rule where it takes them.
-template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP>
+// FIXED: the pitch of the tiles that fit it (FwdShape::pitch), 0 for none.
+template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0>
 __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdata *__restrict__ pd,
                                              const LaunchArgs &a, int e0, int e_end, int bx0, int by0, int bz0,
                                              int ex, int ey, int ez, int lane, bool align4 = false)
@@ -180,7 +181,8 @@ __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdat
             t = min(t, ft);
         }
         const int lt = (align4 && !GATHER) ? (l & ~3) : l;             // the tile's first column
-        const int wt = (align4 && !GATHER) ? ((r - lt + 3) & ~3) : r - lt;  // its row pitch
+        int wt = (align4 && !GATHER) ? ((r - lt + 3) & ~3) : r - lt;  // its row pitch
+        if (FIXED && wt <= FIXED && FIXED * (t - b) <= TCAP) wt = FIXED;
         const int area = wt * (t - b);
         const int mode = (!valid || r <= l || t <= b) ? kSkip : ((ok && area <= TCAP) ? kTile : kDirect);
         const uint32_t img_base = img * a.img_stride;
@@ -691,7 +693,9 @@ __device__ __forceinline__ int walk_fast(const ProjMeta &M, const LaunchArgs &a,
 // CHUNK < LEN walks the column as LEN / CHUNK unrolled chunks in a rolled loop (fewer
 // values live at once); f then sees k whose low bits are compile-time constants.
 // isc / ib as in walk_fast: f receives idx * isc + ib.
-template <int LEN, int CHUNK = LEN, typename F>
+// PITCH: the target's pitch when it is known (a power of two): the voxel's address is then one
+// shift-add on the ALU pipe instead of a multiply-add on the FMA pipe, which bounds this walk.
+template <int LEN, int CHUNK = LEN, uint32_t PITCH = 0, typename F>
 __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a, float nu, float nw, float Pv,
                                           float Rv, const float *__restrict__ Tk, F &&f, uint32_t isc = 1u,
                                           uint32_t ib = 0u)
@@ -700,7 +704,7 @@ __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a
     const float4 cv = M.cv;
     const int4 rc = M.rect;
     const uint4 tgt = M.tgt;
-    const uint32_t pitch = tgt.x, pitchS = pitch * isc;
+    const uint32_t pitch = PITCH ? PITCH : tgt.x, pitchS = pitch * isc;
     if (!(M.flags.z & 2)) return -1;  // uniform over the projection
     const float y = rcp_screened(nw);
     const float ylo = __fmul_rn(__fmaf_rn(-nw, y, 1.0f), y);
@@ -718,15 +722,19 @@ __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a
         return div_exact2(nv, NB2, Y2, YL2);
     };
     if (M.flags.w) {
-        // inside: every pixel is in the rectangle, idx = bits * pitch + K (mod 2^32)
-        const uint32_t K = (du + tgt.y - base_v * pitch) * isc + ib;
+        // inside: every pixel is in the rectangle, idx = bits * pitch + K (mod 2^32).  There
+        // q >= 2, and floor(q + 1/2) = floor(q - 1/2) + 1: one addition of 2^23 - 1/2, which is a
+        // float, with the sum's ulp 1, gives the pixel's bits minus one (pix_bits2 takes two).
+        // 256 layers of the 768 x 768 x 72 scan: forward 5.99 -> 5.79 ms, backward 5.97 -> 5.71.
+        const uint32_t K = (du + tgt.y - (base_v - 1u) * pitch) * isc + ib;
+        const uint64_t magic1 = f2pack(8388607.5f, 8388607.5f);
 #pragma unroll 1
         for (int c0 = 0; c0 < LEN; c0 += CHUNK) {
 #pragma unroll
             for (int kk = 0; kk < CHUNK; kk += 2) {
                 const int k = c0 + kk;
                 uint32_t b0, b1;
-                u2unpack(pix_bits2(qv(k >> 1), half, magic), b0, b1);
+                u2unpack(addrz2(qv(k >> 1), magic1), b0, b1);
                 f(std::true_type{}, k, true, b0 * pitchS + K);
                 f(std::true_type{}, k + 1, true, b1 * pitchS + K);
             }
@@ -980,6 +988,9 @@ template <int BY_, int NT_, int TC_>
 struct FwdShape {
     static constexpr int by = BY_, nt = NT_, tile = TC_, warps = NT_ / 32, cols = BX * BZ / NT_;
     static constexpr size_t smem = (size_t)(BY_ / 4 * BZ * VSTRIDE + G * TC_) * sizeof(uint32_t);
+    // tiles that fit get this pitch (0: each its own width), as walk_exact's PITCH (192^3 x 18
+    // forward 0.119 -> 0.117 ms, 256 layers of the 768 x 768 x 72 scan 5.79 -> 5.75)
+    static constexpr uint32_t pitch = TC_ >= 2048 ? 64 : 0;
     static_assert(BY_ % 4 == 0 && BY_ <= 16 && BX * BZ % NT_ == 0, "forward brick shape");
 };
 using FwdNarrow = FwdShape<BY, NT, TILE_CAP>;
@@ -1049,7 +1060,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
     const bool bulk = !(reinterpret_cast<uintptr_t>(sum) & 15u) && !(a.det_w & 3u) && !(a.img_stride & 3u);
     auto prepare = [&](int c0, int c1) {
         for (int w = warp; w * G < c1 - c0; w += NW)
-            compute_meta<ARITH, LIST, false, FILTER, TCF>(s_meta + w * G, pd, a, c0 + w * G, c1, x0, y0, z0, BX, BYF, BZ,
+            compute_meta<ARITH, LIST, false, FILTER, TCF, SH::pitch>(s_meta + w * G, pd, a, c0 + w * G, c1, x0, y0, z0, BX, BYF, BZ,
                                                   lane, bulk);
     };
     prepare(e_begin, min(e_end, e_begin + MCAP));
@@ -1118,7 +1129,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 }
                 continue;
             }
-            if constexpr (ARITH == kStrict && !FILTER) if (fl.x == kTile && (fl.z & 2)) {
+            if constexpr (ARITH == kStrict && !FILTER) if (fl.x == kTile && (fl.z & 2) && (!SH::pitch || M.tgt.x == SH::pitch)) {
                 // STRICT into a tile, untilted and screened: n_u and n_w are (c.x*px + c.z*pz) + c.w
                 // (c.y*py is a zero), so the lane coordinate's product in every row is formed once
                 // per projection; walk_exact divides per voxel with the column's reciprocal
@@ -1126,7 +1137,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
                     uint4 quad;
                     // a zero adds nothing to a shared-memory tile; no test for it
-                    walk_exact<BYF, 8>(M, a, nu, nw, Pv, Rv, s_meta[buf + g].T, [&](auto, int k, bool in, uint32_t saddr) {
+                    walk_exact<BYF, 8, SH::pitch>(M, a, nu, nw, Pv, Rv, s_meta[buf + g].T, [&](auto, int k, bool in, uint32_t saddr) {
                         if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
                         const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
                         if (in) red_shared_add(saddr, v);
@@ -1224,10 +1235,10 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 if (M.flags.x == kTile) {
                     uint32_t *tile = s_tile + warp * TCF;
                     const int4 rc = M.rect;
-                    const uint32_t pitch = M.tgt.x;
+                    const uint32_t pitch = M.tgt.x, bytes = (((uint32_t)rc.y + 3u) & ~3u) * 4u;
                     for (int r = lane; r < rc.w; r += 32)
                         bulk_add_u32(sum + M.tgt.z + (uint32_t)(rc.z + r) * a.det_w + (uint32_t)rc.x, tile + r * pitch,
-                                     pitch * 4u);
+                                     bytes);
                     bulk_commit();
                     bulk_wait_read();
                     __syncwarp();
@@ -1243,13 +1254,13 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 if (M.flags.x != kTile) continue;
                 uint32_t *tile = s_tile + g * TCF;
                 const int4 rc = M.rect;
-                const int tw = rc.y, th = rc.w;
+                const int tw = rc.y, th = rc.w, pitch = (int)M.tgt.x;
                 for (int r = warp; r < th; r += NW) {
                     uint32_t *dst = sum + M.tgt.z + (uint32_t)(rc.z + r) * a.det_w + (uint32_t)rc.x;
                     for (int c = lane; c < tw; c += 32) {
-                        const uint32_t v = tile[r * tw + c];
+                        const uint32_t v = tile[r * pitch + c];
                         if (v) {
-                            tile[r * tw + c] = 0u;
+                            tile[r * pitch + c] = 0u;
                             atomicAdd(dst + c, v);
                         }
                     }
