@@ -31,6 +31,7 @@ struct ImageSource {
     virtual uint32_t width() const = 0;
     virtual uint32_t height() const = 0;
     virtual void read(int64_t i, float *dst) = 0;  // width*height floats
+    virtual const float *all() const { return nullptr; }  // every image, when they lie together in memory
 };
 
 // The reference's input: every float32 TIFF of a directory, all of the first file's

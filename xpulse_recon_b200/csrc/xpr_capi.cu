@@ -102,17 +102,20 @@ int xpr_create(int device, uint64_t mem_cap_bytes, xpr_ctx **out)
     if (device < 0 || device >= count) return fail(XPR_ERR_INVALID, "device %d out of range (%d devices)", device, count);
     e = cudaSetDevice(device);
     if (e != cudaSuccess) return cuda_fail(e, "cudaSetDevice");
-    cudaDeviceProp prop;
-    e = cudaGetDeviceProperties(&prop, device);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDeviceProperties");
-    if (prop.major < 10) return fail(XPR_ERR_UNSUPPORTED, "device %d is sm_%d%d; this build targets sm_100a", device, prop.major, prop.minor);
+    // (the three attributes, not cudaGetDeviceProperties: that takes 2 ms)
+    int major = 0, minor = 0, sms = 0;
+    e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
+    if (major < 10) return fail(XPR_ERR_UNSUPPORTED, "device %d is sm_%d%d; this build targets sm_100a", device, major, minor);
     e = xpr::prepare_device_kernels();
     if (e != cudaSuccess) return cuda_fail(e, "kernel attributes");
     xpr_ctx *c = new xpr_ctx();
     c->device = device;
     c->cap = mem_cap_bytes;
     c->dev.device = device;
-    c->dev.sm_count = prop.multiProcessorCount;
+    c->dev.sm_count = sms;
     *out = c;
     return XPR_OK;
 }
