@@ -61,9 +61,9 @@ constexpr uint32_t kMagic = 0x4B000000u;  // float bits of 2^23: bits(fadd_rz(y,
 
 enum Mode : int { kSkip = 0, kTile = 1, kDirect = 2 };
 constexpr int kFiltered = 4;  // a projection walked by the filtered pixel rule (xpr_pixel.cuh)
-// What a pass over a unit's projections walks: all of them (the STRICT contract divides per
-// voxel for tilted ones), the untilted ones up to the first chunk with a tilted one, or all by
-// the filtered pixel rule (STRICT).
+// What a pass over a unit's projections walks: all of them (one reciprocal per voxel for a
+// tilted one in FAST, two divisions in STRICT), the untilted ones up to the first chunk with a
+// tilted one, or all by the filtered pixel rule (STRICT).
 enum Pass : int { kAll = 0, kUntilted = 1, kByFilter = 2 };
 
 // Per-projection constants of one (brick, projection) pair, read by every thread as
@@ -571,7 +571,7 @@ __device__ __forceinline__ int walk_fast(const ProjMeta &M, const LaunchArgs &a,
         return 2;
     }
     if (!TILTED || (M.flags.z & 1)) {
-        const float rw = __frcp_rn(Cw);
+        const float rw = (M.flags.z & 2) ? rcp_screened(Cw) : __frcp_rn(Cw);
         const uint32_t du = fdist(__fmaf_rn(Cu, rw, 0.5f), fb.x);
         const bool in_u = du < fb.y;
         if (!__any_sync(0xffffffffu, in_u)) return 0;
@@ -586,6 +586,15 @@ __device__ __forceinline__ int walk_fast(const ProjMeta &M, const LaunchArgs &a,
             const uint32_t dv0 = __float_as_uint(b0) - fb.z, dv1 = __float_as_uint(b1) - fb.z;
             f(std::false_type{}, k, in_u && (dv0 < fb.w), dv0 * pitchS + K);
             f(std::false_type{}, k + 1, in_u && (dv1 < fb.w), dv1 * pitchS + K);
+        }
+    } else if (M.flags.z & 2) {
+#pragma unroll
+        for (int k = 0; k < LEN; k += 2) {
+            uint32_t bu0, bu1, bv0, bv1;
+            tilted_pair<true>(py[k], py[k + 1], cu, cv, cw, Cu, Cv, Cw, hv, bu0, bu1, bv0, bv1);
+            const uint32_t du0 = bu0 - fb.x, du1 = bu1 - fb.x, dv0 = bv0 - fb.z, dv1 = bv1 - fb.z;
+            f(std::false_type{}, k, (du0 < fb.y) && (dv0 < fb.w), (dv0 * pitch + du0 + tgt.y) * isc + ib);
+            f(std::false_type{}, k + 1, (du1 < fb.y) && (dv1 < fb.w), (dv1 * pitch + du1 + tgt.y) * isc + ib);
         }
     } else {
 #pragma unroll
@@ -615,7 +624,7 @@ __device__ __forceinline__ int walk_fast(const ProjMeta &M, const LaunchArgs &a,
     const uint64_t magic = f2pack(8388608.0f, 8388608.0f);
     if (!TILTED || (M.flags.z & 1)) {
         // untilted: u, w and 1/w are column invariants, v = fma(py, Qv, Rv)
-        const float rw = M.flags.w ? rcp_screened(Cw) : __frcp_rn(Cw);
+        const float rw = (M.flags.z & 2) ? rcp_screened(Cw) : __frcp_rn(Cw);
         const float Qv = __fmul_rn(M.cv.y, rw), Rv = __fmaf_rn(Cv, rw, hv);
         const uint64_t Q2 = f2pack(Qv, Qv), R2 = f2pack(Rv, Rv);
         const uint32_t du = fdist(__fmaf_rn(Cu, rw, 0.5f), fb.x);
@@ -669,6 +678,20 @@ __device__ __forceinline__ int walk_fast(const ProjMeta &M, const LaunchArgs &a,
             f(std::true_type{}, k + 1, true, bv1 * pitch + bu1 + Ku);
         }
         return 2;
+    }
+    if (M.flags.z & 2) {
+#pragma unroll
+        for (int k = 0; k < LEN; k += 2) {
+            uint64_t bu, bv;
+            tilted_pair<true>(py2[k >> 1], kp, bu, bv);
+            uint32_t bu0, bu1, bv0, bv1;
+            u2unpack(bu, bu0, bu1);
+            u2unpack(bv, bv0, bv1);
+            const uint32_t du0 = bu0 - fb.x, du1 = bu1 - fb.x, dv0 = bv0 - fb.z, dv1 = bv1 - fb.z;
+            f(std::false_type{}, k, (du0 < fb.y) && (dv0 < fb.w), dv0 * pitch + du0 + tgt.y);
+            f(std::false_type{}, k + 1, (du1 < fb.y) && (dv1 < fb.w), dv1 * pitch + du1 + tgt.y);
+        }
+        return 1;
     }
 #pragma unroll
     for (int k = 0; k < LEN; k += 2) {
@@ -999,8 +1022,9 @@ constexpr size_t kFwdSmem = FwdNarrow::smem;
 
 // The forward of brick `brick` (x fastest, then z, then y) against entries [e_begin, e_end).
 // A kUntilted pass stops in front of the first chunk of projections that has a tilted one and
-// returns that chunk's first entry (else the run's end), from which a kByFilter pass continues:
-// two passes, each with its own registers (in one loop both spilled).
+// returns that chunk's first entry (else the run's end), from which another pass continues:
+// two passes, each with its own registers (in one loop both spilled: FAST on 256 layers of the
+// 768 x 768 x 72 scan forward 4.93 ms, backward 5.36; in two 4.49 and 4.18).
 template <int ARITH, bool LIST, int PASS, typename SH>
 __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uint32_t *__restrict__ sum,
                                              const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
@@ -1008,7 +1032,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                                               int bricks_z, uint32_t *smem, ProjMeta *s_meta)
 {
     constexpr bool TILTED = PASS != kUntilted, FILTER = PASS == kByFilter;
-    static_assert(ARITH == kStrict || PASS == kAll, "FAST walks all projections in one pass");
+    static_assert(ARITH == kStrict || !FILTER, "the filtered rule serves the STRICT contract");
     constexpr int BYF = SH::by, NTF = SH::nt, TCF = SH::tile, NW = SH::warps, CPT = SH::cols;
     // fixed-point values [BYF / 4][BZ][VSTRIDE]: layers 4m .. 4m + 3 of (x, z) are adjacent
     // words, so a thread reads four of its column's voxels with one 128-bit load
@@ -1280,7 +1304,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
 // walks the tilted projections by the filtered pixel rule (384^3, three tilted modules, 36
 // projections: 5.82 ms with two divisions per voxel, 3.50 ms), at a cost of 2 to 4 % for the
 // untilted ones in the same kernel, which one module therefore does not pay.  FAST, whose
-// tilted walk needs one reciprocal per voxel, gains nothing from the rule (2.49 ms, 3.78 with it).
+// tilted walk needs one reciprocal per voxel, loses by the rule (2.27 ms, 3.78 with it).
 template <int ARITH, bool LIST, bool MULTI, typename SH = FwdNarrow>
 __device__ __forceinline__ void forward_unit(const float *__restrict__ vol, uint32_t *__restrict__ sum,
                                              const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
@@ -1288,26 +1312,39 @@ __device__ __forceinline__ void forward_unit(const float *__restrict__ vol, uint
                                              uint32_t *smem, ProjMeta *s_meta)
 {
     const int e0 = (int)split * (int)a.per_split, e1 = min((int)a.n_entries, e0 + (int)a.per_split);
-    if constexpr (ARITH == kStrict && MULTI) {
-        const int stop = forward_bricks<kStrict, LIST, kUntilted, SH>(vol, sum, pd, a, brick, e0, e1, bricks_x, bricks_z,
-                                                                      smem, s_meta);
+    if constexpr (ARITH == kFast || MULTI) {
+        const int stop = forward_bricks<ARITH, LIST, kUntilted, SH>(vol, sum, pd, a, brick, e0, e1, bricks_x, bricks_z,
+                                                                    smem, s_meta);
         if (stop < e1) {
             __syncthreads();
-            forward_bricks<kStrict, LIST, kByFilter, SH>(vol, sum, pd, a, brick, stop, e1, bricks_x, bricks_z, smem, s_meta);
+            forward_bricks<ARITH, LIST, ARITH == kFast ? kAll : kByFilter, SH>(vol, sum, pd, a, brick, stop, e1, bricks_x,
+                                                                              bricks_z, smem, s_meta);
         }
     } else {
         forward_bricks<ARITH, LIST, kAll, SH>(vol, sum, pd, a, brick, e0, e1, bricks_x, bricks_z, smem, s_meta);
     }
 }
 
-template <int ARITH, bool LIST, bool MULTI, typename SH>
+template <bool LIST, bool MULTI, typename SH>
 __global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
     k_forward_tiled(const float *__restrict__ vol, uint32_t *__restrict__ sum, const xpr_projdata *__restrict__ pd,
                     const LaunchArgs a, int bricks_x, int bricks_z)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ ProjMeta s_meta[MCAP];
-    forward_unit<ARITH, LIST, MULTI, SH>(vol, sum, pd, a, blockIdx.x, blockIdx.y, bricks_x, bricks_z, smem, s_meta);
+    forward_unit<kStrict, LIST, MULTI, SH>(vol, sum, pd, a, blockIdx.x, blockIdx.y, bricks_x, bricks_z, smem, s_meta);
+}
+
+// The FAST contract's, with its arguments read in place (the copies that indexing them in a plain
+// parameter makes cost its register-bound walk 8 %, 4.88 -> 4.49 ms; the STRICT walk gains nothing)
+template <bool LIST, typename SH>
+__global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
+    k_forward_fast(const float *__restrict__ vol, uint32_t *__restrict__ sum, const xpr_projdata *__restrict__ pd,
+                   const __grid_constant__ LaunchArgs a, int bricks_x, int bricks_z)
+{
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ ProjMeta s_meta[MCAP];
+    forward_unit<kFast, LIST, false, SH>(vol, sum, pd, a, blockIdx.x, blockIdx.y, bricks_x, bricks_z, smem, s_meta);
 }
 
 // the forward shape of each contract's single-problem kernel
@@ -1428,7 +1465,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                                                 uint32_t brick, int bricks_x, int bricks_z, ProjMeta *s_meta)
 {
     constexpr bool TILTED = PASS != kUntilted, FILTER = PASS == kByFilter;
-    static_assert(ARITH == kStrict || PASS == kAll, "FAST walks all projections in one pass");
+    static_assert(ARITH == kStrict || !FILTER, "the filtered rule serves the STRICT contract");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int b = (int)brick;
     const int bxi = b % bricks_x;
@@ -1554,11 +1591,12 @@ __device__ __forceinline__ void backward_unit(float *__restrict__ vol, const voi
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
                                               uint32_t brick, int bricks_x, int bricks_z, ProjMeta *s_meta)
 {
-    if constexpr (ARITH == kStrict && MULTI) {
-        if (backward_bricks<kStrict, LIST, NANSKIP, kUntilted, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta))
+    if constexpr (ARITH == kFast || MULTI) {
+        if (backward_bricks<ARITH, LIST, NANSKIP, kUntilted, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta))
             return;
         __syncthreads();
-        backward_bricks<kStrict, LIST, NANSKIP, kByFilter, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta);
+        backward_bricks<ARITH, LIST, NANSKIP, ARITH == kFast ? kAll : kByFilter, DT, CB>(vol, ratio, pd, a, brick, bricks_x,
+                                                                                        bricks_z, s_meta);
     } else {
         backward_bricks<ARITH, LIST, NANSKIP, kAll, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta);
     }
@@ -1597,29 +1635,29 @@ __device__ __forceinline__ void store_any(void *p, uint64_t i, float v)
 template <int DT>
 __device__ __forceinline__ void load4(const void *p, uint64_t q, float (&v)[4])  // elements 4 q .. 4 q + 3
 {
-    if (DT == kF32) {
+    if constexpr (DT == kF32) {
         const float4 a = ((const float4 *)p)[q];
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-        return;
-    }
-    const uint2 a = ((const uint2 *)p)[q];
-    const uint32_t h[4] = {a.x & 0xffffu, a.x >> 16, a.y & 0xffffu, a.y >> 16};
+    } else {
+        const uint2 a = ((const uint2 *)p)[q];
+        const uint32_t h[4] = {a.x & 0xffffu, a.x >> 16, a.y & 0xffffu, a.y >> 16};
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        v[k] = DT == kBF16 ? __uint_as_float(h[k] << 16) : __half2float(__ushort_as_half((unsigned short)h[k]));
+        for (int k = 0; k < 4; ++k)
+            v[k] = DT == kBF16 ? __uint_as_float(h[k] << 16) : __half2float(__ushort_as_half((unsigned short)h[k]));
+    }
 }
 template <int DT>
 __device__ __forceinline__ void store4(void *p, uint64_t q, const float (&v)[4])
 {
-    if (DT == kF32) {
+    if constexpr (DT == kF32) {
         ((float4 *)p)[q] = make_float4(v[0], v[1], v[2], v[3]);
-        return;
-    }
-    uint32_t h[4];
+    } else {
+        uint32_t h[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-        h[k] = DT == kBF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v[k])) : __half_as_ushort(__float2half_rn(v[k]));
-    ((uint2 *)p)[q] = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+        for (int k = 0; k < 4; ++k)
+            h[k] = DT == kBF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v[k])) : __half_as_ushort(__float2half_rn(v[k]));
+        ((uint2 *)p)[q] = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+    }
 }
 __device__ __forceinline__ float std_max(float a, float b) { return (a < b) ? b : a; }
 // whether a buffer of `dt` elements can be accessed four at a time
@@ -2101,12 +2139,12 @@ cudaError_t prepare_device_kernels()
     const int smem = (int)kFwdSmem;
     using FwdFn = void (*)(const float *, uint32_t *, const xpr_projdata *, const LaunchArgs, int, int);
     const struct { FwdFn f; size_t smem; } fns[] = {
-        {k_forward_tiled<kStrict, false, false, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
-        {k_forward_tiled<kStrict, true, false, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
-        {k_forward_tiled<kStrict, false, true, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
-        {k_forward_tiled<kStrict, true, true, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
-        {k_forward_tiled<kFast, false, false, FwdShapeOf<kFast>>, FwdShapeOf<kFast>::smem},
-        {k_forward_tiled<kFast, true, false, FwdShapeOf<kFast>>, FwdShapeOf<kFast>::smem}};
+        {k_forward_tiled<false, false, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
+        {k_forward_tiled<true, false, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
+        {k_forward_tiled<false, true, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
+        {k_forward_tiled<true, true, FwdShapeOf<kStrict>>, FwdShapeOf<kStrict>::smem},
+        {k_forward_fast<false, FwdShapeOf<kFast>>, FwdShapeOf<kFast>::smem},
+        {k_forward_fast<true, FwdShapeOf<kFast>>, FwdShapeOf<kFast>::smem}};
     for (const auto &f : fns) {
         e = cudaFuncSetAttribute(f.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
         if (e != cudaSuccess) return e;
@@ -2148,15 +2186,16 @@ static cudaError_t forward_tiled(const float *vol, uint32_t *sum, const xpr_proj
     if (a.n_entries > 0 && bricks > 0) {
         dim3 grid((unsigned)bricks, splits);
         const bool list = a.list_mvp != nullptr;
-        if constexpr (AR == kStrict) {
-            if (a.modules > 1) {  // MULTI (forward_unit)
-                if (list) k_forward_tiled<AR, true, true, SH><<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
-                else k_forward_tiled<AR, false, true, SH><<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
-                return cudaGetLastError();
-            }
+        if constexpr (AR == kFast) {
+            auto *f = list ? k_forward_fast<true, SH> : k_forward_fast<false, SH>;
+            f<<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
+        } else if (a.modules > 1) {  // MULTI (forward_unit)
+            auto *f = list ? k_forward_tiled<true, true, SH> : k_forward_tiled<false, true, SH>;
+            f<<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
+        } else {
+            auto *f = list ? k_forward_tiled<true, false, SH> : k_forward_tiled<false, false, SH>;
+            f<<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
         }
-        if (list) k_forward_tiled<AR, true, false, SH><<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
-        else k_forward_tiled<AR, false, false, SH><<<grid, SH::nt, SH::smem, s>>>(vol, sum, pd, a, bx, bz);
         return cudaGetLastError();
     }
     return cudaSuccess;
