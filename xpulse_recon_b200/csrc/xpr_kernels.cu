@@ -81,6 +81,8 @@ struct __align__(16) ProjMeta {
     uint4 tgt;                            // {pitch, off, img_base, projection index}
     int4 flags;                           // {mode, lanes across z, kind, inside (no bounds tests)}; kind: bit 0
                                           //  untilted, bit 1 walk_exact's screen passed; or kFiltered
+    float4 in0, in1;                      // STRICT, inside and screened: {cu.x, cu.z, cu.w, cw.x}, {cw.z, cw.w, cv.x,
+    uint4 in2;                            //  cv.z}, {cv.w, K0, pitch, 0}: all that walk_inside reads
     float T[16];                          // STRICT: c_v.y * py of the brick's layers (the reference's rounding)
 };
 
@@ -96,7 +98,8 @@ struct __align__(16) ProjMeta {
 template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0>
 __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdata *__restrict__ pd,
                                              const LaunchArgs &a, int e0, int e_end, int bx0, int by0, int bz0,
-                                             int ex, int ey, int ez, int lane, bool align4 = false)
+                                             int ex, int ey, int ez, int lane, bool align4 = false,
+                                             uint32_t tile_s = 0u)
 {
     const int g = lane >> 3, c = lane & 7;
     const int entry = e0 + g;
@@ -241,6 +244,15 @@ __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdat
             }
         }
         M.flags = make_int4(mode, fabsf(cw0) > fabsf(cw2), kind, inside);
+        if (ARITH == kStrict && !FILTER) {
+            // a column's address constant is bits(u) * isc + K0 (walk_inside): the forward's in bytes
+            // of the shared window, with the tile of the entry's place in its group of G
+            const uint32_t isc = GATHER ? 1u : 4u, ib = GATHER ? 0u : tile_s + (uint32_t)(g * TCAP) * 4u;
+            const uint32_t base_v = kMagic + (uint32_t)(b + (int)a.row_off_f) - 1u;
+            M.in0 = make_float4(cu0, cu2, cu3, cw0);
+            M.in1 = make_float4(cw2, cw3, cv0, cv2);
+            M.in2 = make_uint4(__float_as_uint(cv3), (off - (kMagic + (uint32_t)l) - base_v * pitch) * isc + ib, pitch, 0u);
+        }
     }
 }
 
@@ -744,26 +756,6 @@ __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a
         const uint64_t nv = add2(add2(add2(P2, (m & 1) ? T4.y : T4.x), R2), W2);
         return div_exact2(nv, NB2, Y2, YL2);
     };
-    if (M.flags.w) {
-        // inside: every pixel is in the rectangle, idx = bits * pitch + K (mod 2^32).  There
-        // q >= 2, and floor(q + 1/2) = floor(q - 1/2) + 1: one addition of 2^23 - 1/2, which is a
-        // float, with the sum's ulp 1, gives the pixel's bits minus one (pix_bits2 takes two).
-        // 256 layers of the 768 x 768 x 72 scan: forward 5.99 -> 5.79 ms, backward 5.97 -> 5.71.
-        const uint32_t K = (du + tgt.y - (base_v - 1u) * pitch) * isc + ib;
-        const uint64_t magic1 = f2pack(8388607.5f, 8388607.5f);
-#pragma unroll 1
-        for (int c0 = 0; c0 < LEN; c0 += CHUNK) {
-#pragma unroll
-            for (int kk = 0; kk < CHUNK; kk += 2) {
-                const int k = c0 + kk;
-                uint32_t b0, b1;
-                u2unpack(addrz2(qv(k >> 1), magic1), b0, b1);
-                f(std::true_type{}, k, true, b0 * pitchS + K);
-                f(std::true_type{}, k + 1, true, b1 * pitchS + K);
-            }
-        }
-        return 2;
-    }
     const bool in_u = (du < (uint32_t)rc.y) && (qu != -0.5f);
     if (!__any_sync(0xffffffffu, in_u)) return 0;
     const uint32_t K = (du + tgt.y) * isc + ib;
@@ -784,6 +776,42 @@ __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a
         }
     }
     return 1;
+}
+
+// walk_exact where the whole brick lies inside the viewport, from the record compute_meta made
+// for it: nu, nw, Pv, Rv as there, cvw = c_v.w, K0 and pitch from the record.  f(k, idx) gets the
+// target index times isc (plus the record's base).  There q >= 2, and floor(q + 1/2) =
+// floor(q - 1/2) + 1: one addition of 2^23 - 1/2, which is a float, with the sum's ulp 1, gives
+// the pixel's bits minus one (pix_bits2 takes two): 256 layers of the 768 x 768 x 72 scan
+// forward 5.99 -> 5.79 ms, backward 5.97 -> 5.71.
+template <int LEN, int CHUNK, uint32_t PITCH, uint32_t ISC, typename F>
+__device__ __forceinline__ void walk_inside(float nu, float nw, float Pv, float Rv, float cvw, uint32_t K0,
+                                            uint32_t pitch, const float *__restrict__ Tk, F &&f)
+{
+    static_assert(CHUNK % 4 == 0 && LEN % CHUNK == 0, "columns are walked four voxels at a time");
+    const uint32_t pitchS = (PITCH ? PITCH : pitch) * ISC;
+    const float y = rcp_screened(nw);
+    const float ylo = __fmul_rn(__fmaf_rn(-nw, y, 1.0f), y);
+    const uint32_t K = pix_bits(div_exact(nu, -nw, y, ylo)) * ISC + K0;
+    const uint64_t P2 = f2pack(Pv, Pv), R2 = f2pack(Rv, Rv), W2 = f2pack(cvw, cvw);
+    const uint64_t Y2 = f2pack(y, y), YL2 = f2pack(ylo, ylo), NB2 = f2pack(-nw, -nw);
+    const uint64_t magic1 = f2pack(8388607.5f, 8388607.5f);
+#pragma unroll 1
+    for (int c0 = 0; c0 < LEN; c0 += CHUNK) {
+#pragma unroll
+        for (int kk = 0; kk < CHUNK; kk += 4) {
+            const ulonglong2 T4 = reinterpret_cast<const ulonglong2 *>(Tk)[(c0 + kk) >> 2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = c0 + kk + 2 * h;
+                const uint64_t nv = add2(add2(add2(P2, h ? T4.y : T4.x), R2), W2);
+                uint32_t b0, b1;
+                u2unpack(addrz2(div_exact2(nv, NB2, Y2, YL2), magic1), b0, b1);
+                f(k, b0 * pitchS + K);
+                f(k + 1, b1 * pitchS + K);
+            }
+        }
+    }
 }
 
 // The STRICT contract's own pixel of the voxel at (px, py, pz) by the matrix m, relative to the
@@ -1085,7 +1113,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
     auto prepare = [&](int c0, int c1) {
         for (int w = warp; w * G < c1 - c0; w += NW)
             compute_meta<ARITH, LIST, false, FILTER, TCF, SH::pitch>(s_meta + w * G, pd, a, c0 + w * G, c1, x0, y0, z0, BX, BYF, BZ,
-                                                  lane, bulk);
+                                                  lane, bulk, (uint32_t)__cvta_generic_to_shared(s_tile));
     };
     prepare(e_begin, min(e_end, e_begin + MCAP));
     if (!__syncthreads_or(any)) return e_end;   // an all-zero brick adds nothing
@@ -1105,8 +1133,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
         for (int g = 0; g < G; ++g) {
             // a register copy: the walk's shared-memory atomics would otherwise force the
             // metadata to be re-read from shared memory for every column
-            const ProjMeta M = s_meta[buf + g];
-            const int4 fl = M.flags;
+            const int4 fl = s_meta[buf + g].flags;
             if (fl.x == kSkip) continue;
             uint32_t *tile = s_tile + g * TCF;
             // the tile's shared-window address: the tile walks below hand f the atomic's
@@ -1114,6 +1141,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
             const uint32_t tile_s = (uint32_t)__cvta_generic_to_shared(tile);
             const bool orx = fl.y;
             if constexpr (ARITH == kFast) if (fl.x == kTile) {
+                const ProjMeta M = s_meta[buf + g];
                 // FAST into a tile: one lane coordinate is the thread's for all of its columns,
                 // so its share of the column numerators C = fma(c.x, px, c.w) + c.z * pz is
                 // computed once per projection
@@ -1153,6 +1181,49 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 }
                 continue;
             }
+            if constexpr (ARITH == kStrict && !FILTER)
+                if (fl.x == kTile && fl.w && (fl.z & 3) == 3 && (!SH::pitch || s_meta[buf + g].in2.z == SH::pitch)) {
+                // STRICT into a tile, untilted, screened and inside: n_u and n_w are
+                // (c.x*px + c.z*pz) + c.w (c.y*py is a zero), so the lane coordinate's product in
+                // every row is formed once per projection; walk_inside divides per voxel with the
+                // column's reciprocal
+                const float4 i0 = s_meta[buf + g].in0, i1 = s_meta[buf + g].in1;
+                const uint4 i2 = s_meta[buf + g].in2;
+                auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
+                    uint4 quad;
+                    // a zero adds nothing to a shared-memory tile; no test for it
+                    walk_inside<BYF, 8, SH::pitch, 4u>(nu, nw, Pv, Rv, __uint_as_float(i2.x), i2.y, i2.z, s_meta[buf + g].T,
+                                                       [&](int k, uint32_t saddr) {
+                        if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
+                        red_shared_add(saddr, (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x));
+                    });
+                };
+                if (orx) {
+                    const float pz = pos<kStrict>(a.vmin[2] + z0 + lane, a.voxel[2], a.origin[2]);
+                    const float Bu = __fmul_rn(i0.y, pz), Bw = __fmul_rn(i1.x, pz), Rv = __fmul_rn(i1.w, pz);
+#pragma unroll 1
+                    for (int j = 0; j < CPT; ++j) {
+                        const int cx = warp + NW * j;
+                        const float px = pos<kStrict>(a.vmin[0] + x0 + cx, a.voxel[0], a.origin[0]);
+                        splat(reinterpret_cast<const uint4 *>(s_val + lane * VSTRIDE + 4 * cx),
+                              __fadd_rn(__fadd_rn(__fmul_rn(i0.x, px), Bu), i0.z),
+                              __fadd_rn(__fadd_rn(__fmul_rn(i0.w, px), Bw), i1.y), __fmul_rn(i1.z, px), Rv);
+                    }
+                } else {
+                    const float px = pos<kStrict>(a.vmin[0] + x0 + lane, a.voxel[0], a.origin[0]);
+                    const float Au = __fmul_rn(i0.x, px), Aw = __fmul_rn(i0.w, px), Pv = __fmul_rn(i1.z, px);
+#pragma unroll 1
+                    for (int j = 0; j < CPT; ++j) {
+                        const int cz = warp + NW * j;
+                        const float pz = pos<kStrict>(a.vmin[2] + z0 + cz, a.voxel[2], a.origin[2]);
+                        splat(reinterpret_cast<const uint4 *>(s_val + cz * VSTRIDE + 4 * lane),
+                              __fadd_rn(__fadd_rn(Au, __fmul_rn(i0.y, pz)), i0.z),
+                              __fadd_rn(__fadd_rn(Aw, __fmul_rn(i1.x, pz)), i1.y), Pv, __fmul_rn(i1.w, pz));
+                    }
+                }
+                continue;
+            }
+            const ProjMeta M = s_meta[buf + g];
             if constexpr (ARITH == kStrict && !FILTER) if (fl.x == kTile && (fl.z & 2) && (!SH::pitch || M.tgt.x == SH::pitch)) {
                 // STRICT into a tile, untilted and screened: n_u and n_w are (c.x*px + c.z*pz) + c.w
                 // (c.y*py is a zero), so the lane coordinate's product in every row is formed once
@@ -1476,6 +1547,8 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
     // thread = the voxel column (x0 + lane, z0 + warp), layers y0 .. y0 + CB
     const int ax = a.vmin[0] + x0 + lane, az = a.vmin[2] + z0 + warp;
 
+    const float px = pos<ARITH>(ax, a.voxel[0], a.origin[0]), pz = pos<ARITH>(az, a.voxel[2], a.origin[2]);
+
     // the column's y positions are the same for every thread: kept in shared memory
     // (read as broadcasts), which leaves the registers to the sums and the gathers in flight
     __shared__ __align__(16) uint64_t py[CB / 2];  // in pairs {py[2m], py[2m + 1]}
@@ -1555,6 +1628,23 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                     walk_filtered<CB, false>(M, a, pd, fx, fz, ax, ay, az, 1u, 0u, get, put);
                 }
                 continue;
+            }
+            if constexpr (ARITH == kStrict) {
+                const int4 fl = M.flags;
+                if (fl.w && (fl.z & 3) == 3) {
+                    const float4 i0 = M.in0, i1 = M.in1;
+                    const uint4 i2 = M.in2;
+                    walk_inside<CB, CB, 0u, 1u>(
+                        __fadd_rn(__fadd_rn(__fmul_rn(i0.x, px), __fmul_rn(i0.y, pz)), i0.z),
+                        __fadd_rn(__fadd_rn(__fmul_rn(i0.w, px), __fmul_rn(i1.x, pz)), i1.y), __fmul_rn(i1.z, px),
+                        __fmul_rn(i1.w, pz), __uint_as_float(i2.x), i2.y, i2.z, M.T, [&](int k, uint32_t idx) {
+                            rb[k] = load_ratio_bits<DT>(ratio, idx);
+                            if (k == CB / 2 - 1) consume(0);
+                        });
+                    if (!NANSKIP) ++n_inside;
+                    consume(CB / 2);
+                    continue;
+                }
             }
             const int walked = walk_column<ARITH, CB, TILTED>(M, a, ax, az, py, M.T, [&](auto inside, int k, bool in, uint32_t idx) {
                 rb[k] = 0u;
