@@ -81,8 +81,8 @@ struct __align__(16) ProjMeta {
     uint4 tgt;                            // {pitch, off, img_base, projection index}
     int4 flags;                           // {mode, lanes across z, kind, inside (no bounds tests)}; kind: bit 0
                                           //  untilted, bit 1 walk_exact's screen passed; or kFiltered
-    float4 in0, in1;                      // STRICT, inside and screened: {cu.x, cu.z, cu.w, cw.x}, {cw.z, cw.w, cv.x,
-    uint4 in2;                            //  cv.z}, {cv.w, K0, pitch, 0}: all that walk_inside reads
+    float4 in0, in1;                      // untilted, screened and inside: {cu.x, cu.z, cu.w, cw.x}, {cw.z, cw.w,
+    uint4 in2;                            //  cv.x, cv.z}, {cv.w, K0, pitch, cv.y}: all that the inside walks read
     float T[16];                          // STRICT: c_v.y * py of the brick's layers (the reference's rounding)
 };
 
@@ -244,14 +244,16 @@ __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdat
             }
         }
         M.flags = make_int4(mode, fabsf(cw0) > fabsf(cw2), kind, inside);
-        if (ARITH == kStrict && !FILTER) {
-            // a column's address constant is bits(u) * isc + K0 (walk_inside): the forward's in bytes
+        if (!FILTER) {
+            // a column's address constant is bits(u) * isc + K0 (the inside walks): the forward's in bytes
             // of the shared window, with the tile of the entry's place in its group of G
             const uint32_t isc = GATHER ? 1u : 4u, ib = GATHER ? 0u : tile_s + (uint32_t)(g * TCAP) * 4u;
-            const uint32_t base_v = kMagic + (uint32_t)(b + (int)a.row_off_f) - 1u;
+            // (FAST's coordinate has the row offset subtracted; STRICT's bits are the pixel's minus one)
+            const uint32_t base_v = kMagic + (ARITH == kStrict ? (uint32_t)(b + (int)a.row_off_f) - 1u : (uint32_t)b);
             M.in0 = make_float4(cu0, cu2, cu3, cw0);
             M.in1 = make_float4(cw2, cw3, cv0, cv2);
-            M.in2 = make_uint4(__float_as_uint(cv3), (off - (kMagic + (uint32_t)l) - base_v * pitch) * isc + ib, pitch, 0u);
+            M.in2 = make_uint4(__float_as_uint(cv3), (off - (kMagic + (uint32_t)l) - base_v * pitch) * isc + ib, pitch,
+                               __float_as_uint(cv1));
         }
     }
 }
@@ -719,7 +721,8 @@ __device__ __forceinline__ int walk_fast(const ProjMeta &M, const LaunchArgs &a,
     return 1;
 }
 
-// STRICT-contract walk of an untilted column (same calls and return value as walk_fast),
+// STRICT-contract walk of an untilted column with every test of bounds (f as in walk_fast;
+// returns 0, without calling f, when no column of the warp meets the u range, else 1),
 // bit-identical to the reference's per-voxel division: n_v = ((c.x*px + c.y*py) + c.z*pz)
 // + c.w in the reference's order (c.y*py = Tk[k], formed by compute_meta), v = n_v / n_w by
 // div_exact with the column's n_w, and the pixel by pix_bits2.  Returns -1, without calling f, when the projection's operands
@@ -776,6 +779,28 @@ __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a
         }
     }
     return 1;
+}
+
+// The FAST contract's untilted column where the whole brick lies inside the viewport, from the
+// same record (cvy = c_v.y): Cu, Cv, Cw the column's numerators, pair(m) its y positions
+// {py[2m], py[2m + 1]}.  The values are walk_fast's; it reads three vectors of metadata for its
+// seven, and the address constant is ready: 256 layers of the 768 x 768 x 72 scan, bf16 ratios,
+// forward 4.48 -> 4.27 ms, backward 4.18 -> 3.94.
+template <int LEN, uint32_t ISC, typename PY, typename F>
+__device__ __forceinline__ void walk_inside_fast(float Cu, float Cv, float Cw, float cvy, float hv, uint32_t K0,
+                                                 uint32_t pitch, PY &&pair, F &&f)
+{
+    const float rw = rcp_screened(Cw);
+    const uint32_t K = __float_as_uint(__fadd_rz(__fmaf_rn(Cu, rw, 0.5f), 8388608.0f)) * ISC + K0, pitchS = pitch * ISC;
+    const float Qv = __fmul_rn(cvy, rw), Rv = __fmaf_rn(Cv, rw, hv);
+    const uint64_t Q2 = f2pack(Qv, Qv), R2 = f2pack(Rv, Rv), magic = f2pack(8388608.0f, 8388608.0f);
+#pragma unroll
+    for (int k = 0; k < LEN; k += 2) {
+        uint32_t b0, b1;
+        u2unpack(addrz2(fma2(pair(k >> 1), Q2, R2), magic), b0, b1);
+        f(k, b0 * pitchS + K);
+        f(k + 1, b1 * pitchS + K);
+    }
 }
 
 // walk_exact where the whole brick lies inside the viewport, from the record compute_meta made
@@ -1140,6 +1165,46 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
             // address (4 * index + tile_s), formed by their one multiply-add per voxel
             const uint32_t tile_s = (uint32_t)__cvta_generic_to_shared(tile);
             const bool orx = fl.y;
+            if constexpr (ARITH == kFast && !TILTED) if (fl.x == kTile && fl.w) {
+                // FAST into a tile, untilted, screened and inside: as below, from the record.  The
+                // pass with tilted projections keeps walk_fast alone (with both: 2.27 -> 2.36 ms)
+                const float4 i0 = s_meta[buf + g].in0, i1 = s_meta[buf + g].in1;
+                const uint4 i2 = s_meta[buf + g].in2;
+                const float cvw = __uint_as_float(i2.x);
+                auto splat = [&](const uint4 *vals, float Cu, float Cv, float Cw) {
+                    uint4 quad;
+                    walk_inside_fast<BYF, 4u>(Cu, Cv, Cw, __uint_as_float(i2.w), a.half_minus_off, i2.y, i2.z,
+                                              [&](int m) { return f2pack(py[2 * m], py[2 * m + 1]); },
+                                              [&](int k, uint32_t saddr) {
+                        if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
+                        red_shared_add(saddr, (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x));
+                    });
+                };
+                if (orx) {
+                    const float pz = pos<kFast>(a.vmin[2] + z0 + lane, a.voxel[2], a.origin[2]);
+                    const float Pu = __fmul_rn(i0.y, pz), Pv = __fmul_rn(i1.w, pz), Pw = __fmul_rn(i1.x, pz);
+#pragma unroll 1
+                    for (int j = 0; j < CPT; ++j) {
+                        const int cx = warp + NW * j;
+                        const float px = pos<kFast>(a.vmin[0] + x0 + cx, a.voxel[0], a.origin[0]);
+                        splat(reinterpret_cast<const uint4 *>(s_val + lane * VSTRIDE + 4 * cx),
+                              __fadd_rn(__fmaf_rn(i0.x, px, i0.z), Pu), __fadd_rn(__fmaf_rn(i1.z, px, cvw), Pv),
+                              __fadd_rn(__fmaf_rn(i0.w, px, i1.y), Pw));
+                    }
+                } else {
+                    const float px = pos<kFast>(a.vmin[0] + x0 + lane, a.voxel[0], a.origin[0]);
+                    const float Au = __fmaf_rn(i0.x, px, i0.z), Av = __fmaf_rn(i1.z, px, cvw), Aw = __fmaf_rn(i0.w, px, i1.y);
+#pragma unroll 1
+                    for (int j = 0; j < CPT; ++j) {
+                        const int cz = warp + NW * j;
+                        const float pz = pos<kFast>(a.vmin[2] + z0 + cz, a.voxel[2], a.origin[2]);
+                        splat(reinterpret_cast<const uint4 *>(s_val + cz * VSTRIDE + 4 * lane),
+                              __fadd_rn(Au, __fmul_rn(i0.y, pz)), __fadd_rn(Av, __fmul_rn(i1.w, pz)),
+                              __fadd_rn(Aw, __fmul_rn(i1.x, pz)));
+                    }
+                }
+                continue;
+            }
             if constexpr (ARITH == kFast) if (fl.x == kTile) {
                 const ProjMeta M = s_meta[buf + g];
                 // FAST into a tile: one lane coordinate is the thread's for all of its columns,
@@ -1638,6 +1703,29 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                         __fadd_rn(__fadd_rn(__fmul_rn(i0.x, px), __fmul_rn(i0.y, pz)), i0.z),
                         __fadd_rn(__fadd_rn(__fmul_rn(i0.w, px), __fmul_rn(i1.x, pz)), i1.y), __fmul_rn(i1.z, px),
                         __fmul_rn(i1.w, pz), __uint_as_float(i2.x), i2.y, i2.z, M.T, [&](int k, uint32_t idx) {
+                            rb[k] = load_ratio_bits<DT>(ratio, idx);
+                            if (k == CB / 2 - 1) consume(0);
+                        });
+                    if (!NANSKIP) ++n_inside;
+                    consume(CB / 2);
+                    continue;
+                }
+            }
+            if constexpr (ARITH == kFast && !TILTED) {
+                if (M.flags.w) {
+                    const float4 i0 = M.in0, i1 = M.in1;
+                    const uint4 i2 = M.in2;
+                    ulonglong2 p4 = make_ulonglong2(0ull, 0ull);
+                    walk_inside_fast<CB, 1u>(
+                        __fadd_rn(__fmaf_rn(i0.x, px, i0.z), __fmul_rn(i0.y, pz)),
+                        __fadd_rn(__fmaf_rn(i1.z, px, __uint_as_float(i2.x)), __fmul_rn(i1.w, pz)),
+                        __fadd_rn(__fmaf_rn(i0.w, px, i1.y), __fmul_rn(i1.x, pz)), __uint_as_float(i2.w),
+                        a.half_minus_off, i2.y, i2.z,
+                        [&](int m) {
+                            if (!(m & 1)) p4 = reinterpret_cast<const ulonglong2 *>(py)[m >> 1];
+                            return (m & 1) ? p4.y : p4.x;
+                        },
+                        [&](int k, uint32_t idx) {
                             rb[k] = load_ratio_bits<DT>(ratio, idx);
                             if (k == CB / 2 - 1) consume(0);
                         });
