@@ -83,8 +83,19 @@ struct __align__(16) ProjMeta {
                                           //  untilted, bit 1 walk_exact's screen passed; or kFiltered
     float4 in0, in1;                      // untilted, screened and inside: {cu.x, cu.z, cu.w, cw.x}, {cw.z, cw.w,
     uint4 in2;                            //  cv.x, cv.z}, {cv.w, K0, pitch, cv.y}: all that the inside walks read
-    float T[16];                          // STRICT: c_v.y * py of the brick's layers (the reference's rounding)
 };
+template <int LEN>
+struct ProjMetaT : ProjMeta {
+    float T[LEN];                         // c_v.y * py of the brick's layers (the reference's rounding)
+};
+// T has the brick's layers and FAST goes without it: a narrow batch CTA with 16 floats of T (7 KB of
+// metadata) no longer fits four to an SM (48 FAST scans of 96 x 64 x 180: 38.3 ms with four, 40.1
+// with three; 30 STRICT scans of 48 x 32 x 120: 1.15 and 1.24 ms)
+template <int ARITH, int LEN>
+using Meta = std::conditional_t<ARITH == kStrict, ProjMetaT<LEN>, ProjMeta>;
+template <int LEN>
+__device__ __forceinline__ const float *layers(const ProjMetaT<LEN> &M) { return M.T; }
+__device__ __forceinline__ const float *layers(const ProjMeta &) { return nullptr; }
 
 // --------------------------------------------------------------------------------------
 // per-projection metadata: one group of G entries, computed by warp 0
@@ -95,8 +106,8 @@ struct __align__(16) ProjMeta {
 // be a multiple of 4, which keeps the padded rows inside the image rows).
 // FILTER: the projections go by the filtered pixel rule where it takes them.
 // FIXED: the pitch of the tiles that fit it (FwdShape::pitch), 0 for none.
-template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0>
-__device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdata *__restrict__ pd,
+template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0, typename MT>
+__device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__restrict__ pd,
                                              const LaunchArgs &a, int e0, int e_end, int bx0, int by0, int bz0,
                                              int ex, int ey, int ez, int lane, bool align4 = false,
                                              uint32_t tile_s = 0u)
@@ -121,7 +132,7 @@ __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdat
     const float px = __fmaf_rn((float)ix, a.voxel[0], a.origin[0]);
     const float py = __fmaf_rn((float)iy, a.voxel[1], a.origin[1]);
     const float pz = __fmaf_rn((float)iz, a.voxel[2], a.origin[2]);
-    if (ARITH == kStrict && !FILTER) {
+    if constexpr (ARITH == kStrict && !FILTER) {
         // the products c_v.y * py of the STRICT numerator, two layers per lane, rounded as the
         // reference rounds them; walk_exact loads them, so no packed product feeds its sums
         // (the code generator contracts a packed multiply into the packed add that consumes it)
@@ -253,7 +264,7 @@ __device__ __forceinline__ void compute_meta(ProjMeta *s_meta, const xpr_projdat
             M.in0 = make_float4(cu0, cu2, cu3, cw0);
             M.in1 = make_float4(cw2, cw3, cv0, cv2);
             M.in2 = make_uint4(__float_as_uint(cv3), (off - (kMagic + (uint32_t)l) - base_v * pitch) * isc + ib, pitch,
-                               __float_as_uint(cv1));
+                               ARITH == kStrict ? 0u : __float_as_uint(cv1));
         }
     }
 }
@@ -1049,7 +1060,8 @@ __device__ __forceinline__ int walk_column(const ProjMeta &M, const LaunchArgs &
 // forward
 // --------------------------------------------------------------------------------------
 // Whether a chunk's metadata (n <= MCAP entries) has a tilted projection that the brick meets.
-__device__ __forceinline__ bool chunk_tilted(const ProjMeta *s_meta, int n, int lane)
+template <typename M>
+__device__ __forceinline__ bool chunk_tilted(const M *s_meta, int n, int lane)
 {
     static_assert(MCAP == 32, "one entry per lane");
     return __any_sync(0xffffffffu, lane < n && s_meta[lane].flags.x != kSkip && !(s_meta[lane].flags.z & 1));
@@ -1082,7 +1094,7 @@ template <int ARITH, bool LIST, int PASS, typename SH>
 __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uint32_t *__restrict__ sum,
                                              const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
                                               uint32_t brick, int e_begin, int e_end, int bricks_x,
-                                              int bricks_z, uint32_t *smem, ProjMeta *s_meta)
+                                              int bricks_z, uint32_t *smem, Meta<ARITH, SH::by> *s_meta)
 {
     constexpr bool TILTED = PASS != kUntilted, FILTER = PASS == kByFilter;
     static_assert(ARITH == kStrict || !FILTER, "the filtered rule serves the STRICT contract");
@@ -1257,7 +1269,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
                     uint4 quad;
                     // a zero adds nothing to a shared-memory tile; no test for it
-                    walk_inside<BYF, 8, SH::pitch, 4u>(nu, nw, Pv, Rv, __uint_as_float(i2.x), i2.y, i2.z, s_meta[buf + g].T,
+                    walk_inside<BYF, 8, SH::pitch, 4u>(nu, nw, Pv, Rv, __uint_as_float(i2.x), i2.y, i2.z, layers(s_meta[buf + g]),
                                                        [&](int k, uint32_t saddr) {
                         if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
                         red_shared_add(saddr, (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x));
@@ -1297,7 +1309,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
                     uint4 quad;
                     // a zero adds nothing to a shared-memory tile; no test for it
-                    walk_exact<BYF, 8, SH::pitch>(M, a, nu, nw, Pv, Rv, s_meta[buf + g].T, [&](auto, int k, bool in, uint32_t saddr) {
+                    walk_exact<BYF, 8, SH::pitch>(M, a, nu, nw, Pv, Rv, layers(s_meta[buf + g]), [&](auto, int k, bool in, uint32_t saddr) {
                         if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
                         const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
                         if (in) red_shared_add(saddr, v);
@@ -1367,7 +1379,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 } else if (ARITH != kFast && fl.x == kTile) {
                     // a zero adds nothing to a shared-memory tile; no test for it
                     with_py([&](const auto &pyv) {
-                        walk_column<ARITH, BYF, TILTED, (BYF > 8 ? 8 : BYF)>(M, a, ax, az, pyv, s_meta[buf + g].T, [&](auto, int k, bool in, uint32_t idx) {
+                        walk_column<ARITH, BYF, TILTED, (BYF > 8 ? 8 : BYF)>(M, a, ax, az, pyv, layers(s_meta[buf + g]), [&](auto, int k, bool in, uint32_t idx) {
                             if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
                             const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
                             if (in) atomicAdd(&tile[idx], v);
@@ -1375,7 +1387,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                     });
                 } else {
                     with_py([&](const auto &pyv) {
-                        walk_column<ARITH, BYF, TILTED, (BYF > 8 ? 8 : BYF)>(M, a, ax, az, pyv, s_meta[buf + g].T, [&](auto, int k, bool in, uint32_t idx) {
+                        walk_column<ARITH, BYF, TILTED, (BYF > 8 ? 8 : BYF)>(M, a, ax, az, pyv, layers(s_meta[buf + g]), [&](auto, int k, bool in, uint32_t idx) {
                             if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
                             const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
                             if (in & (v != 0u)) atomicAdd(&sum[idx], v);
@@ -1445,7 +1457,7 @@ template <int ARITH, bool LIST, bool MULTI, typename SH = FwdNarrow>
 __device__ __forceinline__ void forward_unit(const float *__restrict__ vol, uint32_t *__restrict__ sum,
                                              const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
                                              uint32_t brick, uint32_t split, int bricks_x, int bricks_z,
-                                             uint32_t *smem, ProjMeta *s_meta)
+                                             uint32_t *smem, Meta<ARITH, SH::by> *s_meta)
 {
     const int e0 = (int)split * (int)a.per_split, e1 = min((int)a.n_entries, e0 + (int)a.per_split);
     if constexpr (ARITH == kFast || MULTI) {
@@ -1467,7 +1479,7 @@ __global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
                     const LaunchArgs a, int bricks_x, int bricks_z)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ ProjMeta s_meta[MCAP];
+    __shared__ Meta<kStrict, SH::by> s_meta[MCAP];
     forward_unit<kStrict, LIST, MULTI, SH>(vol, sum, pd, a, blockIdx.x, blockIdx.y, bricks_x, bricks_z, smem, s_meta);
 }
 
@@ -1479,7 +1491,7 @@ __global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
                    const __grid_constant__ LaunchArgs a, int bricks_x, int bricks_z)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ ProjMeta s_meta[MCAP];
+    __shared__ Meta<kFast, SH::by> s_meta[MCAP];
     forward_unit<kFast, LIST, false, SH>(vol, sum, pd, a, blockIdx.x, blockIdx.y, bricks_x, bricks_z, smem, s_meta);
 }
 
@@ -1598,7 +1610,7 @@ __device__ __forceinline__ float ratio_from_bits(uint32_t b)
 template <int ARITH, bool LIST, bool NANSKIP, int PASS, int DT, int CB>
 __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const void *__restrict__ ratio,
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
-                                                uint32_t brick, int bricks_x, int bricks_z, ProjMeta *s_meta)
+                                                uint32_t brick, int bricks_x, int bricks_z, Meta<ARITH, CB> *s_meta)
 {
     constexpr bool TILTED = PASS != kUntilted, FILTER = PASS == kByFilter;
     static_assert(ARITH == kStrict || !FILTER, "the filtered rule serves the STRICT contract");
@@ -1643,7 +1655,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
         if (PASS == kUntilted && chunk_tilted(s_meta, c1 - c0, lane)) return false;
 #pragma unroll 1
         for (int e = 0; e < c1 - c0; ++e) {
-            const ProjMeta &M = s_meta[e];
+            const Meta<ARITH, CB> &M = s_meta[e];
             if (M.flags.x == kSkip) continue;
             // the column's gathers are issued before any is consumed (all in flight together);
             // an out-of-bounds pair contributes r = 0, and s + 0 == s exactly (s is never -0).
@@ -1702,7 +1714,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                     walk_inside<CB, CB, 0u, 1u>(
                         __fadd_rn(__fadd_rn(__fmul_rn(i0.x, px), __fmul_rn(i0.y, pz)), i0.z),
                         __fadd_rn(__fadd_rn(__fmul_rn(i0.w, px), __fmul_rn(i1.x, pz)), i1.y), __fmul_rn(i1.z, px),
-                        __fmul_rn(i1.w, pz), __uint_as_float(i2.x), i2.y, i2.z, M.T, [&](int k, uint32_t idx) {
+                        __fmul_rn(i1.w, pz), __uint_as_float(i2.x), i2.y, i2.z, layers(M), [&](int k, uint32_t idx) {
                             rb[k] = load_ratio_bits<DT>(ratio, idx);
                             if (k == CB / 2 - 1) consume(0);
                         });
@@ -1734,7 +1746,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                     continue;
                 }
             }
-            const int walked = walk_column<ARITH, CB, TILTED>(M, a, ax, az, py, M.T, [&](auto inside, int k, bool in, uint32_t idx) {
+            const int walked = walk_column<ARITH, CB, TILTED>(M, a, ax, az, py, layers(M), [&](auto inside, int k, bool in, uint32_t idx) {
                 rb[k] = 0u;
                 if (in) rb[k] = load_ratio_bits<DT>(ratio, idx);
                 if constexpr (!decltype(inside)::value) {
@@ -1767,7 +1779,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
 template <int ARITH, bool LIST, bool NANSKIP, bool MULTI, int DT, int CB>
 __device__ __forceinline__ void backward_unit(float *__restrict__ vol, const void *__restrict__ ratio,
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
-                                              uint32_t brick, int bricks_x, int bricks_z, ProjMeta *s_meta)
+                                              uint32_t brick, int bricks_x, int bricks_z, Meta<ARITH, CB> *s_meta)
 {
     if constexpr (ARITH == kFast || MULTI) {
         if (backward_bricks<ARITH, LIST, NANSKIP, kUntilted, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta))
@@ -1785,7 +1797,7 @@ __global__ void __launch_bounds__(NT, 4)
     k_backward_tiled(float *__restrict__ vol, const void *__restrict__ ratio, const xpr_projdata *__restrict__ pd,
                      const LaunchArgs a, int bricks_x, int bricks_z)
 {
-    __shared__ ProjMeta s_meta[MCAP];
+    __shared__ Meta<ARITH, CB> s_meta[MCAP];
     backward_unit<ARITH, LIST, NANSKIP, MULTI, DT, CB>(vol, ratio, pd, a, blockIdx.x, bricks_x, bricks_z, s_meta);
 }
 
@@ -2157,7 +2169,7 @@ __global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
     k_forward_batched(const BatchFwdItem *__restrict__ items, int n_items, uint32_t total_units, uint32_t *ticket)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    __shared__ ProjMeta s_meta[MCAP];
+    __shared__ Meta<ARITH, SH::by> s_meta[MCAP];
     __shared__ LaunchArgs s_a;
     __shared__ uint32_t s_unit;
     __shared__ int s_item;
@@ -2188,7 +2200,7 @@ template <int ARITH, bool MULTI, int DT, int CB>
 __global__ void __launch_bounds__(NT, 4)
     k_backward_batched(const BatchBwdItem *__restrict__ items, int n_items, uint32_t total_units, uint32_t *ticket)
 {
-    __shared__ ProjMeta s_meta[MCAP];
+    __shared__ Meta<ARITH, CB> s_meta[MCAP];
     __shared__ LaunchArgs s_a;
     __shared__ uint32_t s_unit;
     __shared__ int s_item;
