@@ -795,8 +795,8 @@ __device__ __forceinline__ int walk_exact(const ProjMeta &M, const LaunchArgs &a
 // The FAST contract's untilted column where the whole brick lies inside the viewport, from the
 // same record (cvy = c_v.y): Cu, Cv, Cw the column's numerators, pair(m) its y positions
 // {py[2m], py[2m + 1]}.  The values are walk_fast's; it reads three vectors of metadata for its
-// seven, and the address constant is ready: 256 layers of the 768 x 768 x 72 scan, bf16 ratios,
-// forward 4.48 -> 4.27 ms, backward 4.18 -> 3.94.
+// seven, and the address constant is ready: 256 layers of the 768 x 768 x 72 scan, forward
+// 4.48 -> 4.27 ms, backward 4.18 -> 3.90.
 template <int LEN, uint32_t ISC, typename PY, typename F>
 __device__ __forceinline__ void walk_inside_fast(float Cu, float Cv, float Cw, float cvy, float hv, uint32_t K0,
                                                  uint32_t pitch, PY &&pair, F &&f)
