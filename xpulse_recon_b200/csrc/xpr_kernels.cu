@@ -70,7 +70,8 @@ enum Pass : int { kAll = 0, kUntilted = 1, kByFilter = 2 };
 // 16-byte vectors.  Rectangle [u0, u1) x [v0, v1) in buffer coordinates; a pixel
 // (iu, iv) inside it goes to target index (iv - v0) * pitch + (iu - u0) + off, where
 // the target is the shared-memory tile (pitch = tile width, off = 0) or the whole
-// detector buffer (pitch = det_w, off = img_base + v0 * det_w + u0).
+// detector buffer (pitch = det_w, off = img_base + v0 * det_w + u0).  A tile that is flushed by
+// bulk reductions starts on the 4-pixel column at or before u0: its off is the distance.
 struct __align__(16) ProjMeta {
     float4 cu, cv, cw;                    // matrix rows for u, v, w (glm columns c0, c1, c3); kFiltered: the
                                           //  brick-relative rows {c0, cx, cz, cy} (PixRow)
@@ -103,7 +104,9 @@ __device__ __forceinline__ const float *layers(const ProjMeta &) { return nullpt
 // --------------------------------------------------------------------------------------
 // align4: a tile is flushed by 16-byte bulk reductions, so it starts on a 4-pixel column
 // boundary and its rows are padded to a multiple of 4 words (the detector width must then
-// be a multiple of 4, which keeps the padded rows inside the image rows).
+// be a multiple of 4, which keeps the padded rows inside the image rows).  That moves the
+// tile's origin only: the window that a pixel has to lie in still starts at the viewport or
+// the footprint, and the columns in front of it stay zero.
 // FILTER: the projections go by the filtered pixel rule where it takes them.
 // FIXED: the pitch of the tiles that fit it (FwdShape::pitch), 0 for none.
 template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0, typename MT>
@@ -201,9 +204,8 @@ __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__r
         const int mode = (!valid || r <= l || t <= b) ? kSkip : ((ok && area <= TCAP) ? kTile : kDirect);
         const uint32_t img_base = img * a.img_stride;
         const bool tile = (mode == kTile) && !GATHER;
-        if (tile) l = lt;
         const uint32_t pitch = tile ? (uint32_t)wt : a.det_w;
-        const uint32_t off = tile ? 0u : img_base + (uint32_t)b * a.det_w + (uint32_t)l;
+        const uint32_t off = tile ? (uint32_t)(l - lt) : img_base + (uint32_t)b * a.det_w + (uint32_t)l;
         M.cu = make_float4(cu0, cu1, cu2, cu3);
         M.cv = make_float4(cv0, cv1, cv2, cv3);
         M.cw = make_float4(cw0, cw1, cw2, cw3);
@@ -1400,17 +1402,17 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
         __syncthreads();
         if (bulk) {
             // warp g flushes tile g: lane q adds rows q, q + 32, ... to the sums with one bulk
-            // reduction each (rows of `pitch` words from column rect.x, inside the image row),
+            // reduction each (rows of `pitch` words from column rect.x - off, inside the image row),
             // waits until the TMA unit has read them, then the warp zeroes the tile
             if (warp < G) {
                 const ProjMeta &M = s_meta[buf + warp];
                 if (M.flags.x == kTile) {
                     uint32_t *tile = s_tile + warp * TCF;
                     const int4 rc = M.rect;
-                    const uint32_t pitch = M.tgt.x, bytes = (((uint32_t)rc.y + 3u) & ~3u) * 4u;
+                    const uint32_t pitch = M.tgt.x, off = M.tgt.y, bytes = ((off + (uint32_t)rc.y + 3u) & ~3u) * 4u;
                     for (int r = lane; r < rc.w; r += 32)
-                        bulk_add_u32(sum + M.tgt.z + (uint32_t)(rc.z + r) * a.det_w + (uint32_t)rc.x, tile + r * pitch,
-                                     bytes);
+                        bulk_add_u32(sum + M.tgt.z + (uint32_t)(rc.z + r) * a.det_w + (uint32_t)rc.x - off,
+                                     tile + r * pitch, bytes);
                     bulk_commit();
                     bulk_wait_read();
                     __syncwarp();
