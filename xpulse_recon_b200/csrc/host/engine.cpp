@@ -17,6 +17,7 @@
 #include <stdexcept>
 
 #include "../xpr_internal.h"
+#include "arena.h"
 #include "planner.h"
 #include "tiff.h"
 
@@ -58,9 +59,6 @@ struct DevBuf {
     template <class T> T *as() const { return (T *)p; }
     char *at(uint64_t off) const { return (char *)p + off; }
 };
-
-// parts of one allocation start on 256-byte boundaries
-uint64_t aligned(uint64_t n) { return (n + 255) / 256 * 256; }
 
 // a part of a device allocation
 struct Part {
@@ -236,13 +234,14 @@ struct Engine::Impl {
     void preprocess(const Params &p, const std::function<void(int64_t, const void *)> &sink)
     {
         // one device and one page-locked allocation (0.6 and 2 ms each, whatever the size)
-        const uint64_t slot4 = aligned(WH * 4), slot = aligned(WH * iesize);
-        DevBuf dev(ctx, 2 * slot4 + 2 * slot + 8);
-        PinBuf host(ctx, 2 * slot4);
-        char *const raw[2] = {dev.at(0), dev.at(slot4)};
-        char *const out[2] = {dev.at(2 * slot4), dev.at(2 * slot4 + slot)};
-        float *const mm = (float *)dev.at(2 * slot4 + 2 * slot);
-        float *const stage[2] = {(float *)host.at(0), (float *)host.at(slot4)};
+        uint64_t at[6];
+        staging_layout(WH, iesize, available(), at);
+        DevBuf dev(ctx, at[5]);
+        PinBuf host(ctx, 2 * WH * 4);
+        char *const raw[2] = {dev.at(at[0]), dev.at(at[1])};
+        float *const mm = (float *)dev.at(at[2]);
+        char *const out[2] = {dev.at(at[3]), dev.at(at[4])};
+        float *const stage[2] = {(float *)host.at(0), (float *)host.at(WH * 4)};
         Event used[2];
         bool pending[2] = {false, false};
         auto next = [&](int64_t i) {  // image i into staging buffer i % 2, uploaded to raw[i % 2]
@@ -285,7 +284,7 @@ struct Engine::Impl {
     {
         const DeviceInfo *di = context_device(ctx);
         if (!di) throw std::runtime_error(xpr_last_error());
-        float *const mm = (float *)(raw + aligned((uint64_t)P * WH * 4));
+        float *const mm = (float *)(raw + arena_round((uint64_t)P * WH * 4, kArenaPad));
         check(xpr_upload(ctx, raw, src->all(), (uint64_t)P * WH * 4, comp->v()), "upload");
         if (p.normalize) {
             const float init[2] = {FLT_MAX, FLT_MIN};  // data_loader.hpp:12-13
@@ -487,26 +486,19 @@ void Engine::reconstruct()
         std::cout << "Checking GPU memory requierments : " << need / (1024 * 1024) << "Mo" << std::endl;
         const uint64_t available = d.available();
         if (need > available) throw std::runtime_error("Not enough GPU memory");
-        // One device allocation for everything.  Raw images that lie together in host memory go up
-        // in one copy when there is room for them and they are at most kRawAtOnce; larger sets go
-        // image by image through page-locked staging, which overlaps reading and uploading.
+        // One device allocation for everything (resident_layout); larger sets of raw images go image
+        // by image through page-locked staging, which overlaps reading and uploading.
         constexpr uint64_t kRawAtOnce = 256u << 20;
-        const uint64_t raw_bytes = (uint64_t)d.P * WH * 4;
-        // the 32-bit arrays first, so that they stay aligned to their elements when the last bytes
-        // of the device leave no room for the padding
-        const uint64_t bytes[5] = {nvol * 4, Pc * WH * 4, (uint64_t)(S * Pc * M) * PDB, sep ? Pc * WH * d.rsize : 0,
-                                   (uint64_t)(S * Pc) * WH * d.iesize};
-        uint64_t at[6] = {0}, packed = 0;
-        for (int k = 0; k < 5; ++k) at[k + 1] = at[k] + aligned(bytes[k]);
-        if (at[5] > available)
-            for (int k = 0; k < 5; ++k) at[k + 1] = (packed += bytes[k]);
-        const uint64_t used = at[5], raw_part = aligned(raw_bytes) + 8;
-        const bool at_once = d.src->all() && raw_bytes <= kRawAtOnce && used + raw_part <= available;
-        DevBuf dev(d.ctx, used + (at_once ? raw_part : 0));
-        const Part vol{dev.at(at[0])}, sum{dev.at(at[1])}, pd{dev.at(at[2])}, ratio{dev.at(at[3])}, img{dev.at(at[4])};
+        const uint64_t bytes[5] = {nvol * 4, Pc * WH * 4, (uint64_t)(S * Pc * M) * PDB,
+                                   (uint64_t)(S * Pc) * WH * d.iesize, sep ? Pc * WH * d.rsize : 0};
+        const ResidentLayout lay = resident_layout(bytes, d.iesize, WH, d.src->all() ? (uint64_t)d.P * WH * 4 : 0,
+                                                   kRawAtOnce, available);
+        DevBuf dev(d.ctx, lay.total);
+        const Part vol{dev.at(lay.at[0])}, sum{dev.at(lay.at[1])}, pd{dev.at(lay.at[2])}, img{dev.at(lay.at[3])},
+            ratio{dev.at(lay.at[4])};
         std::cout << "Pre-processing images..." << std::flush;
-        if (at_once) {
-            d.preprocess_all(p, dev.at(used), img.p);
+        if (lay.at_once) {
+            d.preprocess_all(p, dev.at(lay.raw), img.p);
         } else {
             d.preprocess(p, [&](int64_t i, const void *dimg) {
                 if (i / S >= Pc) return;  // the kernels use the first Pc angles of a sub-iteration
