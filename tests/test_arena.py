@@ -1,6 +1,6 @@
 """Offsets inside the engine's device allocations (csrc/host/arena.h), checked on the CPU: every
 part on a boundary of its elements for odd image sizes and every pair of storage types, no more
-bytes than the parts have when memory is short."""
+bytes than the parts have when memory is short, and raw images only where there is room to spare."""
 import ctypes as C
 import os
 import shutil
@@ -13,9 +13,9 @@ CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "xpulse_re
 SOURCE = """
 #include "arena.h"
 using u64 = unsigned long;
-extern "C" int resident(const u64 *bytes, u64 elem, u64 pixels, u64 raw, u64 limit, u64 avail, u64 *out)
+extern "C" int resident(const u64 *bytes, u64 elem, u64 pixels, u64 raw, u64 limit, u64 margin, u64 avail, u64 *out)
 {
-    xpr::ResidentLayout l = xpr::resident_layout((const uint64_t *)bytes, elem, pixels, raw, limit, avail);
+    xpr::ResidentLayout l = xpr::resident_layout((const uint64_t *)bytes, elem, pixels, raw, limit, margin, avail);
     for (int k = 0; k < 6; ++k) out[k] = l.at[k];
     out[6] = l.raw;
     out[7] = l.total;
@@ -61,12 +61,12 @@ def test_resident_parts(arena, elem, ratio, width, height, per, sit):
     for avail in [sum(sizes) + k for k in range(0, 3 * 1280 + 2 * stage)] + [BIG]:
         out = (C.c_ulong * 8)()
         once = arena.resident((C.c_ulong * 5)(*sizes), C.c_ulong(elem), C.c_ulong(wh), C.c_ulong(raw), C.c_ulong(BIG),
-                              C.c_ulong(avail), out)
+                              C.c_ulong(64 << 20), C.c_ulong(avail), out)
         at, total = list(out)[:6], out[7]
         check_parts(at, sizes, elems)
         assert total <= avail
         if once:
-            assert out[6] % 256 == 0 and out[6] >= at[5] and total >= out[6] + raw + 8
+            assert avail == BIG and out[6] % 256 == 0 and out[6] >= at[5] and total >= out[6] + raw + 8
         else:
             # what is left takes the two images in flight whenever the bare sums do
             left = avail - total
@@ -75,6 +75,19 @@ def test_resident_parts(arena, elem, ratio, width, height, per, sit):
                 check_parts(s, [4 * wh, 4 * wh, 8, elem * wh, elem * wh], [4, 4, 4, elem, elem])
                 assert s[5] <= left
     assert once
+
+
+def test_raw_images_leave_a_margin(arena):
+    sizes, wh = [4096, 1024, 80, 4096, 0], 256
+    raw = 16 * wh * 4
+    need = 4096 + 1024 + 256 + 4096 + raw + 8
+    for avail, limit, expected in [(need + 1000, raw, 1), (need + 999, raw, 0), (need + 1000, raw - 1, 0), (BIG, raw, 1)]:
+        out = (C.c_ulong * 8)()
+        assert arena.resident((C.c_ulong * 5)(*sizes), C.c_ulong(4), C.c_ulong(wh), C.c_ulong(raw), C.c_ulong(limit),
+                              C.c_ulong(1000), C.c_ulong(avail), out) == expected
+    # images that do not lie together
+    assert arena.resident((C.c_ulong * 5)(*sizes), C.c_ulong(4), C.c_ulong(wh), C.c_ulong(0), C.c_ulong(BIG),
+                          C.c_ulong(0), C.c_ulong(BIG), out) == 0
 
 
 @pytest.mark.gpu

@@ -41,10 +41,11 @@ struct ResidentLayout {
 };
 
 // Raw images that lie together in host memory go up in one copy when they are at most `raw_limit`
-// bytes and fit.  Otherwise the images go up one by one, and what that takes for the two in flight
-// stays free here.
+// bytes and leave `margin` bytes free: they stay allocated for the whole run, and the device needs
+// some room of its own (allocation granularity, kernels loaded at their first launch).  Otherwise
+// the images go up one by one, and what that takes for the two in flight stays free here.
 inline ResidentLayout resident_layout(const uint64_t bytes[5], uint64_t img_elem, uint64_t pixels, uint64_t raw_bytes,
-                                      uint64_t raw_limit, uint64_t available)
+                                      uint64_t raw_limit, uint64_t margin, uint64_t available)
 {
     const uint64_t elem[5] = {4, 4, 4, img_elem, 2};
     ResidentLayout l{};
@@ -53,7 +54,7 @@ inline ResidentLayout resident_layout(const uint64_t bytes[5], uint64_t img_elem
     const bool padded = arena_layout(bytes, elem, 5, available > stage[5] ? available - stage[5] : 0, l.at);
     const uint64_t raw_part = arena_round(raw_bytes, kArenaPad) + 8;
     l.raw = arena_round(l.at[5], kArenaPad);
-    l.at_once = padded && raw_bytes && raw_bytes <= raw_limit && l.raw + raw_part <= available;
+    l.at_once = padded && raw_bytes && raw_bytes <= raw_limit && l.raw + raw_part + margin <= available;
     l.total = l.at_once ? l.raw + raw_part : l.at[5];
     return l;
 }

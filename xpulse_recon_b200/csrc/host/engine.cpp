@@ -43,6 +43,13 @@ struct DevBuf {
     uint64_t bytes = 0;
     DevBuf() = default;
     DevBuf(xpr_ctx *ctx, uint64_t n) : c(ctx), bytes(n) { check(xpr_alloc(ctx, n ? n : 4, &p), "device allocation"); }
+    // null when there is no such block
+    static DevBuf attempt(xpr_ctx *ctx, uint64_t n)
+    {
+        DevBuf b;
+        if (xpr_alloc(ctx, n, &b.p) == XPR_OK) { b.c = ctx; b.bytes = n; }
+        return b;
+    }
     DevBuf(DevBuf &&o) noexcept : c(o.c), p(o.p), bytes(o.bytes) { o.p = nullptr; }
     DevBuf &operator=(DevBuf &&o) noexcept
     {
@@ -488,12 +495,19 @@ void Engine::reconstruct()
         if (need > available) throw std::runtime_error("Not enough GPU memory");
         // One device allocation for everything (resident_layout); larger sets of raw images go image
         // by image through page-locked staging, which overlaps reading and uploading.
-        constexpr uint64_t kRawAtOnce = 256u << 20;
+        constexpr uint64_t kRawAtOnce = 256u << 20, kMargin = 64u << 20;
         const uint64_t bytes[5] = {nvol * 4, Pc * WH * 4, (uint64_t)(S * Pc * M) * PDB,
                                    (uint64_t)(S * Pc) * WH * d.iesize, sep ? Pc * WH * d.rsize : 0};
-        const ResidentLayout lay = resident_layout(bytes, d.iesize, WH, d.src->all() ? (uint64_t)d.P * WH * 4 : 0,
-                                                   kRawAtOnce, available);
-        DevBuf dev(d.ctx, lay.total);
+        auto layout = [&](uint64_t raw_bytes) {
+            return resident_layout(bytes, d.iesize, WH, raw_bytes, kRawAtOnce, kMargin, available);
+        };
+        ResidentLayout lay = layout(d.src->all() ? (uint64_t)d.P * WH * 4 : 0);
+        DevBuf dev;
+        if (lay.at_once) {
+            dev = DevBuf::attempt(d.ctx, lay.total);
+            if (!dev.p) lay = layout(0);  // no such block: without the raw images
+        }
+        if (!dev.p) dev = DevBuf(d.ctx, lay.total);
         const Part vol{dev.at(lay.at[0])}, sum{dev.at(lay.at[1])}, pd{dev.at(lay.at[2])}, img{dev.at(lay.at[3])},
             ratio{dev.at(lay.at[4])};
         std::cout << "Pre-processing images..." << std::flush;
