@@ -305,6 +305,7 @@ struct Engine::Impl {
         }
         check_cuda(launch_preprocess_reorder((const float *)raw, img, idt, WH, (uint32_t)(S * Pc), (uint32_t)S, (uint32_t)Pc,
                                              p.normalize ? 1 : 0, mm, p.mlog ? 1 : 0, *di, comp->s), "preprocess");
+        comp->sync();  // not in the iterations' seconds, and its errors before "Ok."
     }
 
     // n bytes of device memory to host memory: straight into page-locked memory, otherwise
