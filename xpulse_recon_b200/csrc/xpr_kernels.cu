@@ -992,6 +992,9 @@ __device__ __forceinline__ void walk_literal(const ProjMeta &M, const LaunchArgs
     }
 }
 
+// `inside` of a walk that divides per voxel: tests of bounds, but bound by the FMA pipe
+struct Divides : std::false_type {};
+
 // Column walker.  For the voxel column (ax, az) and y-positions py[0..LEN) (in pairs
 // py2[m] = {py[2m], py[2m + 1]}), calls
 // f(inside, k, in, idx) with idx the target index of ProjMeta.  Untilted projections
@@ -1051,7 +1054,7 @@ __device__ __forceinline__ int walk_column(const ProjMeta &M, const LaunchArgs &
                 const float nw = num_strict(cw, px, py, pz);
                 const uint32_t du = (uint32_t)(__float2int_rz(roundf(__fdiv_rn(nu, nw))) - rc.x);
                 const uint32_t dv = (uint32_t)(__float2int_rz(roundf(__fsub_rn(__fdiv_rn(nv, nw), off))) - rc.z);
-                f(std::false_type{}, k, (du < (uint32_t)rc.y) && (dv < (uint32_t)rc.w), dv * pitch + du + tgt.y);
+                f(Divides{}, k, (du < (uint32_t)rc.y) && (dv < (uint32_t)rc.w), dv * pitch + du + tgt.y);
             }
         }
     }
@@ -1575,12 +1578,20 @@ __global__ void k_pad_items(float *vol, uint32_t *sum, const void *ratio, const 
 // The stored bits of ratio element i (zero-extended for the 16-bit types) and their
 // value: a gather returns raw bits so that an out-of-bounds pair can keep 0 (the bits
 // of +0.0 in every type) without a select after the conversion.
-// The address is written as a shift and a 64-bit add, which run on the ALU pipe.  As an array
-// index it was a widening multiply-add: 2.8 cycles per gather of the FMA pipe, which the exact
-// walk keeps busy (256 layers of the 768 x 768 x 72 scan, STRICT: 6.53 -> 6.19 ms).
-template <int DT>
+// ALU: the address is written as a shift and a 64-bit add, which run on the ALU pipe.  As an array
+// index it is a widening multiply-add: 2.8 cycles per gather of the FMA pipe, which the walks
+// inside the viewport and those that divide per voxel keep busy (256 layers of the 768 x 768 x 72
+// scan, STRICT: 6.53 -> 6.19 ms; 384^3 x 36 on one tilted detector 4.04 -> 3.99).  The other walks
+// with tests of bounds have the ALU pipe busy with those and take the array index, one
+// instruction (120 x 90 x 30 on three modules: STRICT 99.2 -> 88.6 us, 92.8 before the shift;
+// 280 x 134 x 38 on two in FAST: 261 -> 229, 247 before; 384^3 x 36 on three: 1.694 -> 1.609 ms).
+template <int DT, bool ALU = true>
 __device__ __forceinline__ uint32_t load_ratio_bits(const void *ratio, uint32_t i)
 {
+    if (!ALU) {
+        if (DT == kF32) return __float_as_uint(__ldg((const float *)ratio + i));
+        return (uint32_t)__ldg((const unsigned short *)ratio + i);
+    }
     uint64_t p;
     asm("{.reg .u64 t;\n\t"
         "cvt.u64.u32 t, %1;\n\t"
@@ -1684,6 +1695,9 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                 auto get = [&](bool in, uint32_t idx) {
                     return in ? load_ratio_bits<DT>(ratio, idx) : (NANSKIP ? kNaNBits<DT> : 0u);
                 };
+                auto get_edge = [&](bool in, uint32_t idx) {
+                    return in ? load_ratio_bits<DT, false>(ratio, idx) : (NANSKIP ? kNaNBits<DT> : 0u);
+                };
                 auto put = [&](int k0, const uint32_t (&w)[8], uint32_t in) {
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
@@ -1704,7 +1718,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                     walk_filtered<CB, true>(M, a, pd, fx, fz, ax, ay, az, 1u, 0u, get, put_inside);
                     ++n_inside;
                 } else {
-                    walk_filtered<CB, false>(M, a, pd, fx, fz, ax, ay, az, 1u, 0u, get, put);
+                    walk_filtered<CB, false>(M, a, pd, fx, fz, ax, ay, az, 1u, 0u, get_edge, put);
                 }
                 continue;
             }
@@ -1750,7 +1764,8 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
             }
             const int walked = walk_column<ARITH, CB, TILTED>(M, a, ax, az, py, layers(M), [&](auto inside, int k, bool in, uint32_t idx) {
                 rb[k] = 0u;
-                if (in) rb[k] = load_ratio_bits<DT>(ratio, idx);
+                constexpr bool alu = decltype(inside)::value || std::is_same_v<decltype(inside), Divides>;
+                if (in) rb[k] = load_ratio_bits<DT, alu>(ratio, idx);
                 if constexpr (!decltype(inside)::value) {
                     if (!NANSKIP && in) n2[k >> 1] += (k & 1) ? 0x10000u : 1u;
                     if (NANSKIP && !in) rb[k] = kNaNBits<DT>;
