@@ -1082,7 +1082,10 @@ struct FwdShape {
     static constexpr int by = BY_, nt = NT_, tile = TC_, warps = NT_ / 32, cols = BX * BZ / NT_;
     static constexpr size_t smem = (size_t)(BY_ / 4 * BZ * VSTRIDE + G * TC_) * sizeof(uint32_t);
     // tiles that fit get this pitch (0: each its own width), as walk_exact's PITCH (192^3 x 18
-    // forward 0.119 -> 0.117 ms, 256 layers of the 768 x 768 x 72 scan 5.79 -> 5.75)
+    // forward 0.119 -> 0.117 ms, 256 layers of the 768 x 768 x 72 scan 5.79 -> 5.75).  Wider ones
+    // (voxels above 1.2 pixels, bricks near the source of a wide cone) take the same walks with
+    // their own pitch: 384^2 x 384 pixels on 36 projections, voxels of 1.45 pixels, 0.673 ms by the
+    // general walk, 0.561 so
     static constexpr uint32_t pitch = TC_ >= 2048 ? 64 : 0;
     static_assert(BY_ % 4 == 0 && BY_ <= 16 && BX * BZ % NT_ == 0, "forward brick shape");
 };
@@ -1264,85 +1267,97 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 continue;
             }
             if constexpr (ARITH == kStrict && !FILTER)
-                if (fl.x == kTile && fl.w && (fl.z & 3) == 3 && (!SH::pitch || s_meta[buf + g].in2.z == SH::pitch)) {
+                if (fl.x == kTile && fl.w && (fl.z & 3) == 3) {
                 // STRICT into a tile, untilted, screened and inside: n_u and n_w are
                 // (c.x*px + c.z*pz) + c.w (c.y*py is a zero), so the lane coordinate's product in
                 // every row is formed once per projection; walk_inside divides per voxel with the
                 // column's reciprocal
                 const float4 i0 = s_meta[buf + g].in0, i1 = s_meta[buf + g].in1;
                 const uint4 i2 = s_meta[buf + g].in2;
-                auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
-                    uint4 quad;
-                    // a zero adds nothing to a shared-memory tile; no test for it
-                    walk_inside<BYF, 8, SH::pitch, 4u>(nu, nw, Pv, Rv, __uint_as_float(i2.x), i2.y, i2.z, layers(s_meta[buf + g]),
-                                                       [&](int k, uint32_t saddr) {
-                        if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
-                        red_shared_add(saddr, (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x));
-                    });
+                auto walk = [&](auto P) {
+                    auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
+                        uint4 quad;
+                        // a zero adds nothing to a shared-memory tile; no test for it
+                        auto add = [&](int k, uint32_t saddr) {
+                            if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
+                            red_shared_add(saddr, (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x));
+                        };
+                        const float cvw = __uint_as_float(i2.x);
+                        const float *T = layers(s_meta[buf + g]);
+                        walk_inside<BYF, 8, decltype(P)::value, 4u>(nu, nw, Pv, Rv, cvw, i2.y, i2.z, T, add);
+                    };
+                    if (orx) {
+                        const float pz = pos<kStrict>(a.vmin[2] + z0 + lane, a.voxel[2], a.origin[2]);
+                        const float Bu = __fmul_rn(i0.y, pz), Bw = __fmul_rn(i1.x, pz), Rv = __fmul_rn(i1.w, pz);
+#pragma unroll 1
+                        for (int j = 0; j < CPT; ++j) {
+                            const int cx = warp + NW * j;
+                            const float px = pos<kStrict>(a.vmin[0] + x0 + cx, a.voxel[0], a.origin[0]);
+                            splat(reinterpret_cast<const uint4 *>(s_val + lane * VSTRIDE + 4 * cx),
+                                  __fadd_rn(__fadd_rn(__fmul_rn(i0.x, px), Bu), i0.z),
+                                  __fadd_rn(__fadd_rn(__fmul_rn(i0.w, px), Bw), i1.y), __fmul_rn(i1.z, px), Rv);
+                        }
+                    } else {
+                        const float px = pos<kStrict>(a.vmin[0] + x0 + lane, a.voxel[0], a.origin[0]);
+                        const float Au = __fmul_rn(i0.x, px), Aw = __fmul_rn(i0.w, px), Pv = __fmul_rn(i1.z, px);
+#pragma unroll 1
+                        for (int j = 0; j < CPT; ++j) {
+                            const int cz = warp + NW * j;
+                            const float pz = pos<kStrict>(a.vmin[2] + z0 + cz, a.voxel[2], a.origin[2]);
+                            splat(reinterpret_cast<const uint4 *>(s_val + cz * VSTRIDE + 4 * lane),
+                                  __fadd_rn(__fadd_rn(Au, __fmul_rn(i0.y, pz)), i0.z),
+                                  __fadd_rn(__fadd_rn(Aw, __fmul_rn(i1.x, pz)), i1.y), Pv, __fmul_rn(i1.w, pz));
+                        }
+                    }
                 };
-                if (orx) {
-                    const float pz = pos<kStrict>(a.vmin[2] + z0 + lane, a.voxel[2], a.origin[2]);
-                    const float Bu = __fmul_rn(i0.y, pz), Bw = __fmul_rn(i1.x, pz), Rv = __fmul_rn(i1.w, pz);
-#pragma unroll 1
-                    for (int j = 0; j < CPT; ++j) {
-                        const int cx = warp + NW * j;
-                        const float px = pos<kStrict>(a.vmin[0] + x0 + cx, a.voxel[0], a.origin[0]);
-                        splat(reinterpret_cast<const uint4 *>(s_val + lane * VSTRIDE + 4 * cx),
-                              __fadd_rn(__fadd_rn(__fmul_rn(i0.x, px), Bu), i0.z),
-                              __fadd_rn(__fadd_rn(__fmul_rn(i0.w, px), Bw), i1.y), __fmul_rn(i1.z, px), Rv);
-                    }
-                } else {
-                    const float px = pos<kStrict>(a.vmin[0] + x0 + lane, a.voxel[0], a.origin[0]);
-                    const float Au = __fmul_rn(i0.x, px), Aw = __fmul_rn(i0.w, px), Pv = __fmul_rn(i1.z, px);
-#pragma unroll 1
-                    for (int j = 0; j < CPT; ++j) {
-                        const int cz = warp + NW * j;
-                        const float pz = pos<kStrict>(a.vmin[2] + z0 + cz, a.voxel[2], a.origin[2]);
-                        splat(reinterpret_cast<const uint4 *>(s_val + cz * VSTRIDE + 4 * lane),
-                              __fadd_rn(__fadd_rn(Au, __fmul_rn(i0.y, pz)), i0.z),
-                              __fadd_rn(__fadd_rn(Aw, __fmul_rn(i1.x, pz)), i1.y), Pv, __fmul_rn(i1.w, pz));
-                    }
-                }
+                if (!SH::pitch || i2.z == SH::pitch) walk(std::integral_constant<uint32_t, SH::pitch>{});
+                else walk(std::integral_constant<uint32_t, 0u>{});
                 continue;
             }
             const ProjMeta M = s_meta[buf + g];
-            if constexpr (ARITH == kStrict && !FILTER) if (fl.x == kTile && (fl.z & 2) && (!SH::pitch || M.tgt.x == SH::pitch)) {
+            if constexpr (ARITH == kStrict && !FILTER) if (fl.x == kTile && (fl.z & 2)) {
                 // STRICT into a tile, untilted and screened: n_u and n_w are (c.x*px + c.z*pz) + c.w
                 // (c.y*py is a zero), so the lane coordinate's product in every row is formed once
                 // per projection; walk_exact divides per voxel with the column's reciprocal
                 const float4 cu = M.cu, cv = M.cv, cw = M.cw;
-                auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
-                    uint4 quad;
-                    // a zero adds nothing to a shared-memory tile; no test for it
-                    walk_exact<BYF, 8, SH::pitch>(M, a, nu, nw, Pv, Rv, layers(s_meta[buf + g]), [&](auto, int k, bool in, uint32_t saddr) {
-                        if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
-                        const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
-                        if (in) red_shared_add(saddr, v);
-                    }, 4u, tile_s);
+                auto walk = [&](auto P) {
+                    auto splat = [&](const uint4 *vals, float nu, float nw, float Pv, float Rv) {
+                        uint4 quad;
+                        // a zero adds nothing to a shared-memory tile; no test for it
+                        auto add = [&](auto, int k, bool in, uint32_t saddr) {
+                            if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
+                            const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
+                            if (in) red_shared_add(saddr, v);
+                        };
+                        const float *T = layers(s_meta[buf + g]);
+                        walk_exact<BYF, 8, decltype(P)::value>(M, a, nu, nw, Pv, Rv, T, add, 4u, tile_s);
+                    };
+                    if (orx) {
+                        const float pz = pos<kStrict>(a.vmin[2] + z0 + lane, a.voxel[2], a.origin[2]);
+                        const float Bu = __fmul_rn(cu.z, pz), Bw = __fmul_rn(cw.z, pz), Rv = __fmul_rn(cv.z, pz);
+#pragma unroll 1
+                        for (int j = 0; j < CPT; ++j) {
+                            const int cx = warp + NW * j;
+                            const float px = pos<kStrict>(a.vmin[0] + x0 + cx, a.voxel[0], a.origin[0]);
+                            splat(reinterpret_cast<const uint4 *>(s_val + lane * VSTRIDE + 4 * cx),
+                                  __fadd_rn(__fadd_rn(__fmul_rn(cu.x, px), Bu), cu.w),
+                                  __fadd_rn(__fadd_rn(__fmul_rn(cw.x, px), Bw), cw.w), __fmul_rn(cv.x, px), Rv);
+                        }
+                    } else {
+                        const float px = pos<kStrict>(a.vmin[0] + x0 + lane, a.voxel[0], a.origin[0]);
+                        const float Au = __fmul_rn(cu.x, px), Aw = __fmul_rn(cw.x, px), Pv = __fmul_rn(cv.x, px);
+#pragma unroll 1
+                        for (int j = 0; j < CPT; ++j) {
+                            const int cz = warp + NW * j;
+                            const float pz = pos<kStrict>(a.vmin[2] + z0 + cz, a.voxel[2], a.origin[2]);
+                            splat(reinterpret_cast<const uint4 *>(s_val + cz * VSTRIDE + 4 * lane),
+                                  __fadd_rn(__fadd_rn(Au, __fmul_rn(cu.z, pz)), cu.w),
+                                  __fadd_rn(__fadd_rn(Aw, __fmul_rn(cw.z, pz)), cw.w), Pv, __fmul_rn(cv.z, pz));
+                        }
+                    }
                 };
-                if (orx) {
-                    const float pz = pos<kStrict>(a.vmin[2] + z0 + lane, a.voxel[2], a.origin[2]);
-                    const float Bu = __fmul_rn(cu.z, pz), Bw = __fmul_rn(cw.z, pz), Rv = __fmul_rn(cv.z, pz);
-#pragma unroll 1
-                    for (int j = 0; j < CPT; ++j) {
-                        const int cx = warp + NW * j;
-                        const float px = pos<kStrict>(a.vmin[0] + x0 + cx, a.voxel[0], a.origin[0]);
-                        splat(reinterpret_cast<const uint4 *>(s_val + lane * VSTRIDE + 4 * cx),
-                              __fadd_rn(__fadd_rn(__fmul_rn(cu.x, px), Bu), cu.w),
-                              __fadd_rn(__fadd_rn(__fmul_rn(cw.x, px), Bw), cw.w), __fmul_rn(cv.x, px), Rv);
-                    }
-                } else {
-                    const float px = pos<kStrict>(a.vmin[0] + x0 + lane, a.voxel[0], a.origin[0]);
-                    const float Au = __fmul_rn(cu.x, px), Aw = __fmul_rn(cw.x, px), Pv = __fmul_rn(cv.x, px);
-#pragma unroll 1
-                    for (int j = 0; j < CPT; ++j) {
-                        const int cz = warp + NW * j;
-                        const float pz = pos<kStrict>(a.vmin[2] + z0 + cz, a.voxel[2], a.origin[2]);
-                        splat(reinterpret_cast<const uint4 *>(s_val + cz * VSTRIDE + 4 * lane),
-                              __fadd_rn(__fadd_rn(Au, __fmul_rn(cu.z, pz)), cu.w),
-                              __fadd_rn(__fadd_rn(Aw, __fmul_rn(cw.z, pz)), cw.w), Pv, __fmul_rn(cv.z, pz));
-                    }
-                }
+                if (!SH::pitch || M.tgt.x == SH::pitch) walk(std::integral_constant<uint32_t, SH::pitch>{});
+                else walk(std::integral_constant<uint32_t, 0u>{});
                 continue;
             }
             // CPT columns per thread; lanes run across the ray so a warp hits distinct pixels
