@@ -51,3 +51,29 @@ def test_footprints_of_every_size(ctx, voxel, modules, arith):
     r.set_ratio_buffer(torch.from_numpy(ratio).cuda())
     r.backward()
     assert_same_bits(d_vol.cpu().numpy(), back)
+
+
+@pytest.mark.parametrize("arith", [O.STRICT, O.FAST])
+@pytest.mark.parametrize("flat", [0, 1, 2])  # modules without tilt
+def test_lists_and_row_windows_of_mixed_modules(ctx, flat, arith):
+    """Index lists in any order, entries repeated, NaN ratios, a box and a row window, on three
+    modules of which some are tilted."""
+    from tests.cases import make_case, oracle_backward, oracle_forward
+    from tests.test_gpu_parity import gpu_backward, gpu_forward
+    c = make_case("modules3_rpy", sit=1, seed=3, row_window=(6, 20), box=((3, 2, 1), (58, 27, 60)))
+    pd = c["pd_all"].reshape(-1, c["M"], 20)
+    untilted = make_case("modules2", sit=1)["pd_all"].reshape(-1, 2, 20)
+    for m in range(flat):  # an untilted module's matrix rows, this scan's viewports
+        pd[:, m, :16] = untilted[np.arange(len(pd)) % len(untilted), 0, :16]
+    rng = np.random.default_rng(flat)
+    n, images = 70, 4
+    lists = (rng.integers(0, len(pd) * c["M"], n).astype(np.uint16), rng.integers(0, images, n).astype(np.uint16))
+    np.testing.assert_array_equal(gpu_forward(ctx, c, arith, lists=lists),
+                                  oracle_forward(c, arith, lists=lists, pd=c["pd_all"]))
+    n_img = max(int(lists[1].max()) + 1, c["Pc"])
+    ratio = rng.uniform(-0.3, 0.3, n_img * c["Wd"] * c["rows"]).astype(np.float32)
+    ratio[rng.random(ratio.size) < 0.05] = np.nan
+    for skip in (0, 1):
+        r = ratio if skip else np.nan_to_num(ratio)
+        assert_same_bits(gpu_backward(ctx, c, r, arith, lists=lists, nan_skip=bool(skip)),
+                         oracle_backward(c, r, arith, nan_skip=skip, lists=lists, pd=c["pd_all"]))

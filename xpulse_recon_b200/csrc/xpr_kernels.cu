@@ -107,7 +107,8 @@ __device__ __forceinline__ const float *layers(const ProjMeta &) { return nullpt
 // be a multiple of 4, which keeps the padded rows inside the image rows).  That moves the
 // tile's origin only: the window that a pixel has to lie in still starts at the viewport or
 // the footprint, and the columns in front of it stay zero.
-// FILTER: the projections go by the filtered pixel rule where it takes them.
+// FILTER: tilted projections, and in the forward all, go by the filtered pixel rule where it takes
+// them.
 // FIXED: the pitch of the tiles that fit it (FwdShape::pitch), 0 for none.
 template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0, typename MT>
 __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__restrict__ pd,
@@ -135,7 +136,7 @@ __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__r
     const float px = __fmaf_rn((float)ix, a.voxel[0], a.origin[0]);
     const float py = __fmaf_rn((float)iy, a.voxel[1], a.origin[1]);
     const float pz = __fmaf_rn((float)iz, a.voxel[2], a.origin[2]);
-    if constexpr (ARITH == kStrict && !FILTER) {
+    if constexpr (ARITH == kStrict && (GATHER || !FILTER)) {
         // the products c_v.y * py of the STRICT numerator, two layers per lane, rounded as the
         // reference rounds them; walk_exact loads them, so no packed product feeds its sums
         // (the code generator contracts a packed multiply into the packed add that consumes it)
@@ -217,10 +218,10 @@ __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__r
         const int column = (cu1 == 0.0f) && (cw1 == 0.0f);
         int kind = !valid ? 1 : (ARITH == kStrict && !column) ? 0 : column | ((scr && (wpos || wneg)) << 1);
         if (ARITH == kFast) inside = inside && (kind & 2);  // the inside walks take rcp_screened
-        if (FILTER) {
-            // the filtered rule's coefficients, relative to the brick's first voxel, and its bound
+        if (FILTER && !(GATHER && column)) {
             kind = 0;
-            if (ok && mode != kSkip) {
+            // the filtered rule's coefficients, relative to the brick's first voxel, and its bound
+            if (ok && mode != kSkip && max(r - l, t - b) <= kPixWindow) {  // (pix_bound's first test)
                 const float fu[4] = {cu0, cu1, cu2, cu3}, fv[4] = {cv0, cv1, cv2, cv3}, fw[4] = {cw0, cw1, cw2, cw3};
                 PixBrick k;
                 double n[3] = {cu3, cv3, cw3};
@@ -257,7 +258,7 @@ __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__r
             }
         }
         M.flags = make_int4(mode, fabsf(cw0) > fabsf(cw2), kind, inside);
-        if (!FILTER) {
+        if (!FILTER || (GATHER && column)) {
             // a column's address constant is bits(u) * isc + K0 (the inside walks): the forward's in bytes
             // of the shared window, with the tile of the entry's place in its group of G
             const uint32_t isc = GATHER ? 1u : 4u, ib = GATHER ? 0u : tile_s + (uint32_t)(g * TCAP) * 4u;
@@ -1706,7 +1707,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                     }
                 }
             };
-            if constexpr (FILTER) {
+            if constexpr (FILTER) if (M.flags.z == kFiltered) {
                 auto get = [&](bool in, uint32_t idx) {
                     return in ? load_ratio_bits<DT>(ratio, idx) : (NANSKIP ? kNaNBits<DT> : 0u);
                 };
@@ -1727,9 +1728,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                 };
                 const float fx = (float)lane, fz = (float)warp;
                 const int ay = a.vmin[1] + y0;
-                if (M.flags.z != kFiltered) {
-                    walk_literal<CB>(M, a, pd, ax, ay, az, 1u, 0u, get, put);
-                } else if (M.flags.w && !NANSKIP) {
+                if (M.flags.w && !NANSKIP) {
                     walk_filtered<CB, true>(M, a, pd, fx, fz, ax, ay, az, 1u, 0u, get, put_inside);
                     ++n_inside;
                 } else {
@@ -1807,7 +1806,10 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
     return true;
 }
 
-// MULTI as in forward_unit (384^3, three tilted modules, 36 projections: 4.82 -> 2.83 ms)
+// MULTI as in forward_unit (384^3, three tilted modules, 36 projections: 4.82 -> 2.83 ms).  The
+// second pass walks untilted projections, and tilted ones that the filter does not take, as a kAll
+// pass does: one tilted module of three, 72 projections, 6.01 ms with all by the rule, 4.85 so
+// (5.17 with two divisions for the tilted ones).
 template <int ARITH, bool LIST, bool NANSKIP, bool MULTI, int DT, int CB>
 __device__ __forceinline__ void backward_unit(float *__restrict__ vol, const void *__restrict__ ratio,
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
