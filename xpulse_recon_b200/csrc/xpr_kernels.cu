@@ -61,9 +61,10 @@ constexpr uint32_t kMagic = 0x4B000000u;  // float bits of 2^23: bits(fadd_rz(y,
 
 enum Mode : int { kSkip = 0, kTile = 1, kDirect = 2 };
 constexpr int kFiltered = 4;  // a projection walked by the filtered pixel rule (xpr_pixel.cuh)
+constexpr int kOther = 8;     // one that a pass skips and the next one walks
 // What a pass over a unit's projections walks: all of them (one reciprocal per voxel for a
-// tilted one in FAST, two divisions in STRICT), the untilted ones up to the first chunk with a
-// tilted one, or all by the filtered pixel rule (STRICT).
+// tilted one in FAST, two divisions in STRICT), the untilted ones (forward_bricks and
+// backward_bricks say up to where), or the tilted ones by the filtered pixel rule (STRICT).
 enum Pass : int { kAll = 0, kUntilted = 1, kByFilter = 2 };
 
 // Per-projection constants of one (brick, projection) pair, read by every thread as
@@ -108,13 +109,15 @@ __device__ __forceinline__ const float *layers(const ProjMeta &) { return nullpt
 // tile's origin only: the window that a pixel has to lie in still starts at the viewport or
 // the footprint, and the columns in front of it stay zero.
 // FILTER: tilted projections, and in the forward all, go by the filtered pixel rule where it takes
-// them.
+// them.  UNTILTED: tilted ones are marked kOther.
 // FIXED: the pitch of the tiles that fit it (FwdShape::pitch), 0 for none.
-template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0, typename MT>
+// tilted_until: the forward's kByFilter pass leaves out untilted projections before this entry.
+template <int ARITH, bool LIST, bool GATHER, bool FILTER, int TCAP = TILE_CAP, int FIXED = 0, bool UNTILTED = false,
+          typename MT>
 __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__restrict__ pd,
                                              const LaunchArgs &a, int e0, int e_end, int bx0, int by0, int bz0,
                                              int ex, int ey, int ez, int lane, bool align4 = false,
-                                             uint32_t tile_s = 0u)
+                                             uint32_t tile_s = 0u, int tilted_until = 0)
 {
     const int g = lane >> 3, c = lane & 7;
     const int entry = e0 + g;
@@ -129,6 +132,7 @@ __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__r
     const float cu0 = __ldg(m + 0), cu1 = __ldg(m + 1), cu2 = __ldg(m + 2), cu3 = __ldg(m + 3);
     const float cv0 = __ldg(m + 4), cv1 = __ldg(m + 5), cv2 = __ldg(m + 6), cv3 = __ldg(m + 7);
     const float cw0 = __ldg(m + 12), cw1 = __ldg(m + 13), cw2 = __ldg(m + 14), cw3 = __ldg(m + 15);
+    if (FILTER && !GATHER) valid = valid && !(entry < tilted_until && cu1 == 0.0f && cw1 == 0.0f);
     // corner voxel centres of the brick (nominal extent; partial bricks are covered)
     const int ix = a.vmin[0] + bx0 + ((c & 1) ? ex - 1 : 0);
     const int iy = a.vmin[1] + by0 + ((c & 2) ? ey - 1 : 0);
@@ -257,7 +261,8 @@ __device__ __forceinline__ void compute_meta(MT *s_meta, const xpr_projdata *__r
                 }
             }
         }
-        M.flags = make_int4(mode, fabsf(cw0) > fabsf(cw2), kind, inside);
+        const bool other = UNTILTED && !column;
+        M.flags = make_int4(other ? kSkip : mode, fabsf(cw0) > fabsf(cw2), other && mode != kSkip ? kOther : kind, inside);
         if (!FILTER || (GATHER && column)) {
             // a column's address constant is bits(u) * isc + K0 (the inside walks): the forward's in bytes
             // of the shared window, with the tile of the entry's place in its group of G
@@ -1065,12 +1070,16 @@ __device__ __forceinline__ int walk_column(const ProjMeta &M, const LaunchArgs &
 // --------------------------------------------------------------------------------------
 // forward
 // --------------------------------------------------------------------------------------
-// Whether a chunk's metadata (n <= MCAP entries) has a tilted projection that the brick meets.
+// Whether a chunk's metadata (n <= MCAP entries) has tilted (bit 1) and untilted (bit 0)
+// projections that the brick meets.
 template <typename M>
-__device__ __forceinline__ bool chunk_tilted(const M *s_meta, int n, int lane)
+__device__ __forceinline__ int chunk_kinds(const M *s_meta, int n, int lane)
 {
     static_assert(MCAP == 32, "one entry per lane");
-    return __any_sync(0xffffffffu, lane < n && s_meta[lane].flags.x != kSkip && !(s_meta[lane].flags.z & 1));
+    const int4 fl = s_meta[min(lane, n - 1)].flags;
+    const bool live = fl.x != kSkip, untilted = live && (fl.z & 1);
+    return (__any_sync(0xffffffffu, (live && !untilted) || fl.z == kOther) ? 2 : 0) |
+           (__any_sync(0xffffffffu, untilted) ? 1 : 0);
 }
 
 // Forward brick shapes: 32 x by x 32 voxels, nt threads (cols = 1024 / nt columns of by
@@ -1095,17 +1104,22 @@ using FwdTall = FwdShape<16, 512, 2048>;
 constexpr size_t kFwdSmem = FwdNarrow::smem;
 
 // The forward of brick `brick` (x fastest, then z, then y) against entries [e_begin, e_end).
-// A kUntilted pass stops in front of the first chunk of projections that has a tilted one and
-// returns that chunk's first entry (else the run's end), from which another pass continues:
-// two passes, each with its own registers (in one loop both spilled: FAST on 256 layers of the
-// 768 x 768 x 72 scan forward 4.93 ms, backward 5.36; in two 4.49 and 4.18).
+// Two passes, each with its own registers (in one loop both spilled: FAST on 256 layers of the
+// 768 x 768 x 72 scan forward 4.93 ms, backward 5.36; in two 4.49 and 4.18).  A kUntilted pass
+// returns the first entry of the first chunk of projections with a tilted one (else the run's end),
+// from which the second pass continues on the brick that the first one loaded, and in
+// `tilted_until` the entry up to which it walked the untilted ones: in FAST the same, as the
+// second pass takes both as they come and its metadata is the first's; in STRICT the first chunk
+// whose projections are all tilted.
 template <int ARITH, bool LIST, int PASS, typename SH>
 __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uint32_t *__restrict__ sum,
                                              const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
                                               uint32_t brick, int e_begin, int e_end, int bricks_x,
-                                              int bricks_z, uint32_t *smem, Meta<ARITH, SH::by> *s_meta)
+                                              int bricks_z, uint32_t *smem, Meta<ARITH, SH::by> *s_meta,
+                                              int &tilted_until)
 {
     constexpr bool TILTED = PASS != kUntilted, FILTER = PASS == kByFilter;
+    constexpr bool SECOND = FILTER || (PASS == kAll && ARITH == kFast);
     static_assert(ARITH == kStrict || !FILTER, "the filtered rule serves the STRICT contract");
     constexpr int BYF = SH::by, NTF = SH::nt, TCF = SH::tile, NW = SH::warps, CPT = SH::cols;
     // fixed-point values [BYF / 4][BZ][VSTRIDE]: layers 4m .. 4m + 3 of (x, z) are adjacent
@@ -1122,8 +1136,8 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
     const int x0 = bxi * BX, y0 = byi * BYF, z0 = bzi * BZ;
     const int sx = a.size[0], sy = a.size[1], sz = a.size[2];
 
-    bool any = false;
-    for (int i = threadIdx.x; i < BX * BYF * BZ; i += NTF) {
+    bool any = SECOND;
+    if (!SECOND) for (int i = threadIdx.x; i < BX * BYF * BZ; i += NTF) {
         const int x = i & 31, z = (i >> 5) & 31, y = i >> 10;
         const int gx = x0 + x, gy = y0 + y, gz = z0 + z;
         uint32_t v = 0;
@@ -1131,7 +1145,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
         s_val[((y >> 2) * BZ + z) * VSTRIDE + 4 * x + (y & 3)] = v;
         any |= (v != 0u);
     }
-    for (int i = threadIdx.x; i < G * TCF; i += NTF) s_tile[i] = 0u;
+    if (!SECOND) for (int i = threadIdx.x; i < G * TCF; i += NTF) s_tile[i] = 0u;
     // the column's y positions: registers for 8-layer columns; for 16-layer columns (STRICT,
     // whose exact walk reads only the c_v.y*py products) in shared memory as pairs, for the
     // per-voxel fallback
@@ -1158,22 +1172,34 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
     const bool bulk = !(reinterpret_cast<uintptr_t>(sum) & 15u) && !(a.det_w & 3u) && !(a.img_stride & 3u);
     auto prepare = [&](int c0, int c1) {
         for (int w = warp; w * G < c1 - c0; w += NW)
-            compute_meta<ARITH, LIST, false, FILTER, TCF, SH::pitch>(s_meta + w * G, pd, a, c0 + w * G, c1, x0, y0, z0, BX, BYF, BZ,
-                                                  lane, bulk, (uint32_t)__cvta_generic_to_shared(s_tile));
+            compute_meta<ARITH, LIST, false, FILTER, TCF, SH::pitch, PASS == kUntilted && ARITH == kStrict>(
+                s_meta + w * G, pd, a, c0 + w * G, c1, x0, y0, z0, BX, BYF, BZ, lane, bulk,
+                (uint32_t)__cvta_generic_to_shared(s_tile), tilted_until);
     };
-    prepare(e_begin, min(e_end, e_begin + MCAP));
-    if (!__syncthreads_or(any)) return e_end;   // an all-zero brick adds nothing
+    __shared__ int s_stop;
+    if (PASS == kUntilted && ARITH == kStrict && threadIdx.x == 0) s_stop = e_end;
+    if (!SECOND || FILTER) {
+        prepare(e_begin, min(e_end, e_begin + MCAP));
+        if (!__syncthreads_or(any)) return e_end;   // an all-zero brick adds nothing
+    }
 
-    int stop = e_end;
-    for (int e0 = e_begin; e0 < e_end; e0 += G) {
+    int stop = e_end;  // STRICT: s_stop, which costs no register
+    int e0 = e_begin;
+    for (; e0 < e_end; e0 += G) {
         const int buf = (e0 - e_begin) % MCAP;
         if (buf == 0 && e0 > e_begin) {
             prepare(e0, min(e_end, e0 + MCAP));
             __syncthreads();
         }
-        if (PASS == kUntilted && buf == 0 && chunk_tilted(s_meta, min(MCAP, e_end - e0), lane)) {
-            stop = e0;
-            break;
+        if (PASS == kUntilted && buf == 0) {
+            const int kinds = chunk_kinds(s_meta, min(MCAP, e_end - e0), lane);
+            if constexpr (ARITH == kStrict) {
+                if ((kinds & 2) && threadIdx.x == 0) s_stop = min(s_stop, e0);
+                if (kinds == 2) break;
+            } else if (kinds & 2) {
+                stop = e0;
+                break;
+            }
         }
 #pragma unroll 1
         for (int g = 0; g < G; ++g) {
@@ -1463,6 +1489,11 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
         __syncthreads();
     }
     if (bulk && warp < G) bulk_wait_all();  // the unit's reductions complete before it ends
+    if constexpr (PASS == kUntilted && ARITH == kStrict) {
+        tilted_until = e0;
+        __syncthreads();
+        return s_stop;
+    }
     return stop;
 }
 
@@ -1471,9 +1502,13 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
 // Called by every thread of the CTA; returns with the CTA converged.
 // MULTI (several detector modules, whose mounting errors are what tilts a projection): STRICT
 // walks the tilted projections by the filtered pixel rule (384^3, three tilted modules, 36
-// projections: 5.82 ms with two divisions per voxel, 3.50 ms), at a cost of 2 to 4 % for the
+// projections: 5.81 ms with two divisions per voxel, 3.08 ms), at a cost of 2 to 4 % for the
 // untilted ones in the same kernel, which one module therefore does not pay.  FAST, whose
 // tilted walk needs one reciprocal per voxel, loses by the rule (2.27 ms, 3.78 with it).
+// Against one that loads the brick anew and walks untilted projections among tilted ones by the
+// rule too, the second pass as it is took three tilted modules from 3.52 to 3.08 ms, one tilted
+// module of three (72 projections) from 6.62 to 5.21, and a FAST scan of 100 x 80 x 10 on two
+// tilted ones from 49.0 to 38.1 us.
 template <int ARITH, bool LIST, bool MULTI, typename SH = FwdNarrow>
 __device__ __forceinline__ void forward_unit(const float *__restrict__ vol, uint32_t *__restrict__ sum,
                                              const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
@@ -1481,31 +1516,33 @@ __device__ __forceinline__ void forward_unit(const float *__restrict__ vol, uint
                                              uint32_t *smem, Meta<ARITH, SH::by> *s_meta)
 {
     const int e0 = (int)split * (int)a.per_split, e1 = min((int)a.n_entries, e0 + (int)a.per_split);
+    int tilted_until = 0;
     if constexpr (ARITH == kFast || MULTI) {
         const int stop = forward_bricks<ARITH, LIST, kUntilted, SH>(vol, sum, pd, a, brick, e0, e1, bricks_x, bricks_z,
-                                                                    smem, s_meta);
+                                                                    smem, s_meta, tilted_until);
         if (stop < e1) {
             __syncthreads();
             forward_bricks<ARITH, LIST, ARITH == kFast ? kAll : kByFilter, SH>(vol, sum, pd, a, brick, stop, e1, bricks_x,
-                                                                              bricks_z, smem, s_meta);
+                                                                              bricks_z, smem, s_meta, tilted_until);
         }
     } else {
-        forward_bricks<ARITH, LIST, kAll, SH>(vol, sum, pd, a, brick, e0, e1, bricks_x, bricks_z, smem, s_meta);
+        forward_bricks<ARITH, LIST, kAll, SH>(vol, sum, pd, a, brick, e0, e1, bricks_x, bricks_z, smem, s_meta, tilted_until);
     }
 }
 
 template <bool LIST, bool MULTI, typename SH>
 __global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
     k_forward_tiled(const float *__restrict__ vol, uint32_t *__restrict__ sum, const xpr_projdata *__restrict__ pd,
-                    const LaunchArgs a, int bricks_x, int bricks_z)
+                    const __grid_constant__ LaunchArgs a, int bricks_x, int bricks_z)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ Meta<kStrict, SH::by> s_meta[MCAP];
     forward_unit<kStrict, LIST, MULTI, SH>(vol, sum, pd, a, blockIdx.x, blockIdx.y, bricks_x, bricks_z, smem, s_meta);
 }
 
-// The FAST contract's, with its arguments read in place (the copies that indexing them in a plain
-// parameter makes cost its register-bound walk 8 %, 4.88 -> 4.49 ms; the STRICT walk gains nothing)
+// The FAST contract's.  Both have their arguments read in place (the copies that indexing them in a
+// plain parameter makes cost FAST's register-bound walk 8 %, 4.88 -> 4.49 ms, STRICT's 1 %, and 9 % on
+// one tilted detector)
 template <bool LIST, typename SH>
 __global__ void __launch_bounds__(SH::nt, 1024 / SH::nt)
     k_forward_fast(const float *__restrict__ vol, uint32_t *__restrict__ sum, const xpr_projdata *__restrict__ pd,
@@ -1681,7 +1718,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
         for (int w = warp; w * G < c1 - c0; w += NWB)
             compute_meta<ARITH, LIST, true, FILTER>(s_meta + w * G, pd, a, c0 + w * G, c1, x0, y0, z0, BX, CB, BWD_BZ, lane);
         __syncthreads();
-        if (PASS == kUntilted && chunk_tilted(s_meta, c1 - c0, lane)) return false;
+        if (PASS == kUntilted && (chunk_kinds(s_meta, c1 - c0, lane) & 2)) return false;
 #pragma unroll 1
         for (int e = 0; e < c1 - c0; ++e) {
             const Meta<ARITH, CB> &M = s_meta[e];
@@ -1806,10 +1843,11 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
     return true;
 }
 
-// MULTI as in forward_unit (384^3, three tilted modules, 36 projections: 4.82 -> 2.83 ms).  The
+// MULTI as in forward_unit (384^3, three tilted modules, 36 projections: 4.82 -> 2.73 ms).  The
 // second pass walks untilted projections, and tilted ones that the filter does not take, as a kAll
 // pass does: one tilted module of three, 72 projections, 6.01 ms with all by the rule, 4.85 so
-// (5.17 with two divisions for the tilted ones).
+// (5.17 with two divisions for the tilted ones).  It starts the unit over: handing it the sums cost
+// the first pass registers (454 x 301 x 45 on two untilted modules 1.67 -> 2.07 ms).
 template <int ARITH, bool LIST, bool NANSKIP, bool MULTI, int DT, int CB>
 __device__ __forceinline__ void backward_unit(float *__restrict__ vol, const void *__restrict__ ratio,
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
