@@ -967,37 +967,6 @@ __device__ __forceinline__ void walk_filtered(const ProjMeta &M, const LaunchArg
     }
 }
 
-// The same with the contract's operations for every voxel: projections that the filter does not
-// take (a window above kPixWindow pixels, n_w not positive over the brick, an error
-// bound above kPixMaxE).
-template <int LEN, typename Get, typename Put>
-__device__ __forceinline__ void walk_literal(const ProjMeta &M, const LaunchArgs &a,
-                                             const xpr_projdata *__restrict__ pd, int ax, int ay0, int az,
-                                             uint32_t isc, uint32_t ib, Get &&get, Put &&put)
-{
-    const int4 rc = M.rect;
-    const float *m = pd[M.tgt.w].mvp;
-    const uint32_t pitchS = M.tgt.x * isc, K0 = M.tgt.y * isc + ib;
-#pragma unroll
-    for (int c0 = 0; c0 < LEN; c0 += 8) {
-        uint32_t wd[8];
-        uint32_t inm = 0u;
-#pragma unroll 1
-        for (int kk = 0; kk < 8; ++kk) {
-            uint32_t du, dv;
-            const bool in = literal_pixel(m, pos<kStrict>(ax, a.voxel[0], a.origin[0]),
-                                                 pos<kStrict>(ay0 + c0 + kk, a.voxel[1], a.origin[1]),
-                                                 pos<kStrict>(az, a.voxel[2], a.origin[2]), a, rc, du, dv);
-            const uint32_t x = get(in, dv * pitchS + (du * isc + K0));
-            inm |= in ? 1u << kk : 0u;
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j == kk) wd[j] = x;
-        }
-        put(c0, wd, inm);
-    }
-}
-
 // `inside` of a walk that divides per voxel: tests of bounds, but bound by the FMA pipe
 struct Divides : std::false_type {};
 
@@ -1102,6 +1071,50 @@ struct FwdShape {
 using FwdNarrow = FwdShape<BY, NT, TILE_CAP>;
 using FwdTall = FwdShape<16, 512, 2048>;
 constexpr size_t kFwdSmem = FwdNarrow::smem;
+
+// Where a brick's voxels lie: the position of its first one and the voxel size, as the contract
+// reads them.
+struct BrickGrid {
+    int x, y, z;
+    float vx, vy, vz, ox, oy, oz, row_off;
+};
+
+// One projection of a kByFilter pass that the filter does not take (a window above kPixWindow
+// pixels, n_w not positive over the brick, an error bound above kPixMaxE), by the contract's own
+// operations for every voxel.  A function of its own, called once per brick and projection:
+// inlined, its unrolled divisions made the walks around it spill (untilted projections of
+// 454 x 301 x 45 on two modules 2.22 -> 2.31 ms); rolled up, eight voxels at a time through one
+// division, it took longer (768 x 768 pixels x 36 on three tilted modules, voxels of 4 pixels:
+// 1.24 ms, 1.00 so, 0.90 inlined).
+template <typename SH>
+__device__ __noinline__ void forward_refused(uint32_t *sum, uint32_t val_s, uint32_t tile_s, int4 flags, float4 cu,
+                                             float4 cv, float4 cw, int4 rc, uint4 tgt, BrickGrid b)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll 1
+    for (int j = 0; j < SH::cols; ++j) {
+        const int cx = flags.y ? warp + SH::warps * j : lane, cz = flags.y ? lane : warp + SH::warps * j;
+        const float px = pos<kStrict>(b.x + cx, b.vx, b.ox), pz = pos<kStrict>(b.z + cz, b.vz, b.oz);
+        const uint4 *vals = static_cast<const uint4 *>(__cvta_shared_to_generic(val_s + (cz * VSTRIDE + 4 * cx) * 4u));
+        uint4 quad;
+#pragma unroll 1
+        for (int c0 = 0; c0 < SH::by; c0 += 8)
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {
+                const int k = c0 + kk;
+                const float py = pos<kStrict>(b.y + k, b.vy, b.oy), nw = num_strict(cw, px, py, pz);
+                const uint32_t du = (uint32_t)(__float2int_rz(roundf(__fdiv_rn(num_strict(cu, px, py, pz), nw))) - rc.x);
+                const uint32_t dv = (uint32_t)(__float2int_rz(roundf(__fsub_rn(__fdiv_rn(num_strict(cv, px, py, pz), nw), b.row_off))) - rc.z);
+                if (!(k & 3)) quad = vals[(k >> 2) * (BZ * VSTRIDE / 4)];
+                const uint32_t v = (k & 2) ? ((k & 1) ? quad.w : quad.z) : ((k & 1) ? quad.y : quad.x);
+                if (du < (uint32_t)rc.y && dv < (uint32_t)rc.w && v != 0u) {
+                    const uint32_t idx = dv * tgt.x + du + tgt.y;
+                    if (flags.x == kDirect) atomicAdd(&sum[idx], v);
+                    else red_shared_add(tile_s + 4u * idx, v);
+                }
+            }
+    }
+}
 
 // The forward of brick `brick` (x fastest, then z, then y) against entries [e_begin, e_end).
 // Two passes, each with its own registers (in one loop both spilled: FAST on 256 layers of the
@@ -1342,6 +1355,12 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                 continue;
             }
             const ProjMeta M = s_meta[buf + g];
+            if constexpr (FILTER) if (fl.z != kFiltered) {
+                forward_refused<SH>(sum, (uint32_t)__cvta_generic_to_shared(s_val), tile_s, fl, M.cu, M.cv, M.cw, M.rect, M.tgt,
+                                    BrickGrid{a.vmin[0] + x0, a.vmin[1] + y0, a.vmin[2] + z0, a.voxel[0], a.voxel[1],
+                                              a.voxel[2], a.origin[0], a.origin[1], a.origin[2], a.row_off_f});
+                continue;
+            }
             if constexpr (ARITH == kStrict && !FILTER) if (fl.x == kTile && (fl.z & 2)) {
                 // STRICT into a tile, untilted and screened: n_u and n_w are (c.x*px + c.z*pz) + c.w
                 // (c.y*py is a zero), so the lane coordinate's product in every row is formed once
@@ -1420,8 +1439,7 @@ __device__ __forceinline__ int forward_bricks(const float *__restrict__ vol, uin
                     };
                     const float fx = (float)cx, fz = (float)cz;
                     const uint32_t isc = direct ? 1u : 4u, ib = direct ? 0u : tile_s;
-                    if (fl.z != kFiltered) walk_literal<BYF>(M, a, pd, ax, ay, az, isc, ib, get, put_any);
-                    else if (fl.w && !direct) walk_filtered<BYF, true>(M, a, pd, fx, fz, ax, ay, az, 4u, tile_s, get, put_tile);
+                    if (fl.w && !direct) walk_filtered<BYF, true>(M, a, pd, fx, fz, ax, ay, az, 4u, tile_s, get, put_tile);
                     else walk_filtered<BYF, false>(M, a, pd, fx, fz, ax, ay, az, isc, ib, get, put_any);
                 } else if (ARITH != kFast && fl.x == kTile) {
                     // a zero adds nothing to a shared-memory tile; no test for it
