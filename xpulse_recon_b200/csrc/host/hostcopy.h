@@ -20,4 +20,17 @@ inline void par_memcpy(void *dst, const void *src, size_t n)
     }
 }
 
+// Writes one byte of every page of [dst, dst + n), memory that is about to be overwritten: pages
+// that the caller never touched are mapped by several threads at once, where a copy would map them
+// one by one from its own thread.
+inline void par_touch(void *dst, size_t n)
+{
+    constexpr size_t kPage = 4096;
+    volatile char *p = (volatile char *)dst;
+    const int64_t pages = (int64_t)(n / kPage);
+#pragma omp parallel for schedule(static) num_threads(8)
+    for (int64_t i = 0; i < pages; ++i) p[(size_t)i * kPage] = 0;
+    if (n) p[n - 1] = 0;
+}
+
 }  // namespace xpr
