@@ -353,7 +353,6 @@ __device__ __forceinline__ void mul_rn2v(float &d0, float &d1, float a0, float a
         : "=f"(d0), "=f"(d1)
         : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
-__device__ __forceinline__ float rcp_screened(float b);
 // FAST contract for two voxels of a tilted column: the pixel coordinates' bits
 // fadd_rz(y, 2^23) for u (bu0, bu1) and v (bv0, bv1), with
 // rw = 1/fma(c_w.y, py, C_w), yu = fma(py, c_u.y*rw, fma(C_u, rw, 1/2)),
@@ -457,20 +456,7 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
     return d;
 }
 
-// RN(1 / b) for 2^-60 <= |b| <= 2^60: the hardware's approximation (at most one ulp off) and
-// one Newton step, whose fused residual 1 - b y is exact, so that the step's one rounding gives
-// the correctly rounded reciprocal (Markstein, IBM J. Res. Dev. 34(1), 1990; he excepts divisors
-// whose mantissa is all ones).  Compared with __frcp_rn over all 2^23 mantissas: no difference,
-// all ones included.  The general __frcp_rn takes any b, with its branch and its range checks.
-// With it and four layers per load of the y products: 256 layers of the 768 x 768 x 72 scan
-// forward 6.33 -> 5.99 ms, backward 6.19 -> 5.96 (STRICT); three tilted modules in FAST (one
-// reciprocal per voxel) forward 2.72 -> 2.49 ms, backward 2.78 -> 2.30 (384^3, 36 projections).
-__device__ __forceinline__ float rcp_screened(float b)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    return __fmaf_rn(__fmaf_rn(-b, y, 1.0f), y, y);
-}
+// rcp_screened (xpr_math.cuh) of a register pair
 __device__ __forceinline__ uint64_t rcp_screened2(uint64_t b, uint64_t one)
 {
     float b0, b1, y0, y1;
@@ -894,9 +880,7 @@ __device__ __forceinline__ void walk_filtered(const ProjMeta &M, const LaunchArg
     const float nw = __fmaf_rn(mw.y, fx, __fmaf_rn(mw.z, fz, mw.x));
     const float nv = __fmaf_rn(mv.y, fx, __fmaf_rn(mv.z, fz, mv.x));
     const float nu = __fmaf_rn(mu.y, fx, __fmaf_rn(mu.z, fz, mu.x));
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(nw));
-    y = __fmaf_rn(__fmaf_rn(-nw, y, 1.0f), y, y);
+    const float y = rcp_screened(nw);
     // n / (1 + k e), e the relative change of n_w per layer, as a quadratic in the layer k
     const float e = __fmul_rn(mw.w, y);
     const float V0 = __fmaf_rn(nv, y, C), V1 = __fmaf_rn(-__fmul_rn(nv, y), e, __fmul_rn(mv.w, y)),
@@ -1976,7 +1960,8 @@ __device__ __forceinline__ float p_logf_normal(float x)
 // p_logf_normal of two numbers, two per packed instruction (2.04 cycles of the FMA pipe for the
 // pair; a scalar one takes 1.41): 240 images of 768 x 768, minimum, maximum and preprocessing
 // 443 -> 367 us.  The mantissa's range (above sqrt(2): halved) and the exponent come from one
-// integer addition with its carry, the exponent's float from its bits.
+// integer addition with its carry (the offset reduction common to published logf's), the
+// exponent's float from its bits.
 __device__ __forceinline__ void p_logf_normal2(float &x0, float &x1)
 {
     constexpr uint32_t kHalf = 0x3f3504f4u;  // bits of the smallest mantissa above sqrt(2), halved
