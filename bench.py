@@ -375,8 +375,8 @@ REF_SAMPLE_LAYERS = 128  # the central y-slab both CPU legs time when the whole 
 
 
 def cpu_reference_step_factory(cfg, seconds_target, max_layers=REF_SAMPLE_LAYERS):
-    """The reference's own OpenCL kernels (oracle/_ref, built from its sources) on the host
-    cores: forward + error + backward of a y-slab of the grid against one sub-iteration's
+    """The reference's own OpenCL kernels (oracle/_ref, built from its sources; without them the
+    oracle's restatement of their arithmetic, kind "port") on the host cores: forward + error + backward of a y-slab of the grid against one sub-iteration's
     projections -- the whole grid when it is small (c1), else the central max_layers layers
     (the same sample for cpu_baseline and the reference arm, so that their fixed costs --
     the error step over the whole detector -- weigh the same).  seconds_target only sets
@@ -446,6 +446,11 @@ def run_reference(args, cfg, rank, world):
         emit({"impl": "reference", "unavailable": "the reference runs one reconstruction per process; %s is a "
               "batched / served / out-of-core workload of this library (time its single-problem kernels with "
               "--config c2)" % args.config})
+        return 0
+    from oracle import oracle as O
+    if O.ref_lib() is None:
+        emit({"impl": "reference", "unavailable": "the reference's kernels are not built (oracle/_ref): its sources "
+              "are not here"})
         return 0
     # the cpu_baseline sample (whole small grids once per step; else the central 128-layer slab,
     # thinned to no fewer than 64 layers only if the whole run would take over about five
