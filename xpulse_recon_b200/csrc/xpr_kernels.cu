@@ -1640,6 +1640,8 @@ __global__ void k_pad_items(float *vol, uint32_t *sum, const void *ratio, const 
 // with tests of bounds have the ALU pipe busy with those and take the array index, one
 // instruction (120 x 90 x 30 on three modules: STRICT 99.2 -> 88.6 us, 92.8 before the shift;
 // 280 x 134 x 38 on two in FAST: 261 -> 229, 247 before; 384^3 x 36 on three: 1.694 -> 1.609 ms).
+// The batched kernels, whose registers are full, shift and add in all walks (ALU_EDGES: 17 FAST
+// scans of 130 x 63 x 183 5.36 ms, 5.52 by the index; in STRICT 6.66 and 6.72).
 template <int DT, bool ALU = true>
 __device__ __forceinline__ uint32_t load_ratio_bits(const void *ratio, uint32_t i)
 {
@@ -1675,7 +1677,7 @@ __device__ __forceinline__ float ratio_from_bits(uint32_t b)
 //
 // PASS as in forward_bricks; a kUntilted pass that meets a tilted projection returns false,
 // nothing written, and a kByFilter pass does the unit from its start.
-template <int ARITH, bool LIST, bool NANSKIP, int PASS, int DT, int CB>
+template <int ARITH, bool LIST, bool NANSKIP, int PASS, int DT, int CB, bool ALU_EDGES>
 __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const void *__restrict__ ratio,
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
                                                 uint32_t brick, int bricks_x, int bricks_z, Meta<ARITH, CB> *s_meta)
@@ -1751,7 +1753,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
                     return in ? load_ratio_bits<DT>(ratio, idx) : (NANSKIP ? kNaNBits<DT> : 0u);
                 };
                 auto get_edge = [&](bool in, uint32_t idx) {
-                    return in ? load_ratio_bits<DT, false>(ratio, idx) : (NANSKIP ? kNaNBits<DT> : 0u);
+                    return in ? load_ratio_bits<DT, ALU_EDGES>(ratio, idx) : (NANSKIP ? kNaNBits<DT> : 0u);
                 };
                 auto put = [&](int k0, const uint32_t (&w)[8], uint32_t in) {
 #pragma unroll
@@ -1817,7 +1819,7 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
             }
             const int walked = walk_column<ARITH, CB, TILTED>(M, a, ax, az, py, layers(M), [&](auto inside, int k, bool in, uint32_t idx) {
                 rb[k] = 0u;
-                constexpr bool alu = decltype(inside)::value || std::is_same_v<decltype(inside), Divides>;
+                constexpr bool alu = ALU_EDGES || decltype(inside)::value || std::is_same_v<decltype(inside), Divides>;
                 if (in) rb[k] = load_ratio_bits<DT, alu>(ratio, idx);
                 if constexpr (!decltype(inside)::value) {
                     if (!NANSKIP && in) n2[k >> 1] += (k & 1) ? 0x10000u : 1u;
@@ -1850,19 +1852,19 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
 // pass does: one tilted module of three, 72 projections, 6.01 ms with all by the rule, 4.85 so
 // (5.17 with two divisions for the tilted ones).  It starts the unit over: handing it the sums cost
 // the first pass registers (454 x 301 x 45 on two untilted modules 1.67 -> 2.07 ms).
-template <int ARITH, bool LIST, bool NANSKIP, bool MULTI, int DT, int CB>
+template <int ARITH, bool LIST, bool NANSKIP, bool MULTI, int DT, int CB, bool ALU_EDGES = false>
 __device__ __forceinline__ void backward_unit(float *__restrict__ vol, const void *__restrict__ ratio,
                                               const xpr_projdata *__restrict__ pd, const LaunchArgs &a,
                                               uint32_t brick, int bricks_x, int bricks_z, Meta<ARITH, CB> *s_meta)
 {
     if constexpr (ARITH == kFast || MULTI) {
-        if (backward_bricks<ARITH, LIST, NANSKIP, kUntilted, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta))
+        if (backward_bricks<ARITH, LIST, NANSKIP, kUntilted, DT, CB, ALU_EDGES>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta))
             return;
         __syncthreads();
-        backward_bricks<ARITH, LIST, NANSKIP, ARITH == kFast ? kAll : kByFilter, DT, CB>(vol, ratio, pd, a, brick, bricks_x,
+        backward_bricks<ARITH, LIST, NANSKIP, ARITH == kFast ? kAll : kByFilter, DT, CB, ALU_EDGES>(vol, ratio, pd, a, brick, bricks_x,
                                                                                         bricks_z, s_meta);
     } else {
-        backward_bricks<ARITH, LIST, NANSKIP, kAll, DT, CB>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta);
+        backward_bricks<ARITH, LIST, NANSKIP, kAll, DT, CB, ALU_EDGES>(vol, ratio, pd, a, brick, bricks_x, bricks_z, s_meta);
     }
 }
 
@@ -2294,7 +2296,7 @@ __global__ void __launch_bounds__(NT, 4)
         const uint32_t u = s_unit;
         if (u >= total_units) break;
         const BatchBwdItem &I = items[s_item];
-        backward_unit<ARITH, false, false, MULTI, DT, CB>(I.vol, I.ratio, I.pd, s_a, u - I.unit_begin, I.bricks_x,
+        backward_unit<ARITH, false, false, MULTI, DT, CB, true>(I.vol, I.ratio, I.pd, s_a, u - I.unit_begin, I.bricks_x,
                                                    I.bricks_z, s_meta);
         __syncthreads();
     }
