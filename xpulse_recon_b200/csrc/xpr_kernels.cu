@@ -1641,7 +1641,8 @@ __global__ void k_pad_items(float *vol, uint32_t *sum, const void *ratio, const 
 // instruction (120 x 90 x 30 on three modules: STRICT 99.2 -> 88.6 us, 92.8 before the shift;
 // 280 x 134 x 38 on two in FAST: 261 -> 229, 247 before; 384^3 x 36 on three: 1.694 -> 1.609 ms).
 // The batched kernels, whose registers are full, shift and add in all walks (ALU_EDGES: 17 FAST
-// scans of 130 x 63 x 183 5.36 ms, 5.52 by the index; in STRICT 6.66 and 6.72).
+// scans of 130 x 63 x 183 5.36 ms, 5.52 by the index; in STRICT 6.66 and 6.72), and so does FAST
+// with NaN ratios to skip (100 layers of 500^2 x 40 projections 0.581 and 0.589).
 template <int DT, bool ALU = true>
 __device__ __forceinline__ uint32_t load_ratio_bits(const void *ratio, uint32_t i)
 {
@@ -1819,7 +1820,8 @@ __device__ __forceinline__ bool backward_bricks(float *__restrict__ vol, const v
             }
             const int walked = walk_column<ARITH, CB, TILTED>(M, a, ax, az, py, layers(M), [&](auto inside, int k, bool in, uint32_t idx) {
                 rb[k] = 0u;
-                constexpr bool alu = ALU_EDGES || decltype(inside)::value || std::is_same_v<decltype(inside), Divides>;
+                constexpr bool alu = ALU_EDGES || (ARITH == kFast && NANSKIP) || decltype(inside)::value ||
+                                     std::is_same_v<decltype(inside), Divides>;
                 if (in) rb[k] = load_ratio_bits<DT, alu>(ratio, idx);
                 if constexpr (!decltype(inside)::value) {
                     if (!NANSKIP && in) n2[k >> 1] += (k & 1) ? 0x10000u : 1u;
