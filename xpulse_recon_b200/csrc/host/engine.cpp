@@ -313,14 +313,15 @@ struct Engine::Impl {
     void download_host(void *dst, const void *dsrc, uint64_t n)
     {
         cudaPointerAttributes at{};
-        const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
+        const bool known = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+        const bool pinned = known && at.type == cudaMemoryTypeHost;
         cudaGetLastError();
         // The driver copies pageable memory at 18 GB/s here, page-locking two chunks takes 7 ms: whole
         // calls with a result of 67 MB 7.7 ms so, 14.9 by chunks; of 256 MB 25 and 31.  Into memory
         // that was never touched the driver's copy drops to 4 GB/s (67 MB 18.7 ms, 256 MB 67), unless
         // its pages are mapped first (11.1 and 34).
         if (pinned || n <= (256u << 20)) {
-            if (!pinned && n > (8u << 20)) par_touch(dst, n);
+            if (!known && n > (8u << 20)) par_touch(dst, n);  // (plain host memory only)
             check(xpr_download(ctx, dst, dsrc, n, comp->v()), "download");
             comp->sync();
             return;

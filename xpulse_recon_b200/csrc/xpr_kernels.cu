@@ -82,7 +82,7 @@ struct __align__(16) ProjMeta {
     int4 rect;                            // {u0, u1 - u0, v0, v1 - v0}
     uint4 tgt;                            // {pitch, off, img_base, projection index}
     int4 flags;                           // {mode, lanes across z, kind, inside (no bounds tests)}; kind: bit 0
-                                          //  untilted, bit 1 walk_exact's screen passed; or kFiltered
+                                          //  untilted, bit 1 walk_exact's screen passed; or kFiltered, kOther
     float4 in0, in1;                      // untilted, screened and inside: {cu.x, cu.z, cu.w, cw.x}, {cw.z, cw.w,
     uint4 in2;                            //  cv.x, cv.z}, {cv.w, K0, pitch, cv.y}: all that the inside walks read
 };
