@@ -321,7 +321,7 @@ struct Engine::Impl {
         // that was never touched the driver's copy drops to 4 GB/s (67 MB 18.7 ms, 256 MB 67), unless
         // its pages are mapped first (11.1 and 34).
         if (pinned || n <= (256u << 20)) {
-            if (!known && n > (8u << 20)) par_touch(dst, n);  // (plain host memory only)
+            if (!known && n > (8u << 20)) par_map(dst, n);  // (plain host memory only)
             check(xpr_download(ctx, dst, dsrc, n, comp->v()), "download");
             comp->sync();
             return;
