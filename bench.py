@@ -88,20 +88,20 @@ NOMINAL_FP32_LANES = 148 * 128
 # c2 geometry's central 256-layer slab (150,994,944 voxels, FP32 storage); scaled to a
 # launch by its voxel count for the same geometry
 MEASURED_TRAFFIC_PER_VOXEL = {
-    "strict": {"forward": 716.5e6 / 150994944, "backward": 1212.0e6 / 150994944},
-    "fast": {"forward": 719.7e6 / 150994944, "backward": 1220.9e6 / 150994944},
+    "strict": {"forward": 717.1e6 / 150994944, "backward": 1210.2e6 / 150994944},
+    "fast": {"forward": 716.8e6 / 150994944, "backward": 1220.5e6 / 150994944},
 }
 # executed-work figures of the same captures (profiles/k_*_c2slab.md): issue-active share,
 # l1tex (shared-memory pipe) throughput and thread instructions per (voxel, projection) pair
 MEASURED_PROFILE = {
-    "strict": {"forward": {"issue_active_pct": 69.4, "l1tex_pct": 82.7, "fma_pipe_pct": 57.0,
-                           "thread_inst_per_pair": 12.8, "shared_atomic_replay_pct": 48.6},
-               "backward": {"issue_active_pct": 76.9, "l1tex_pct": 61.6, "fma_pipe_pct": 62.2,
-                            "thread_inst_per_pair": 14.3},
+    "strict": {"forward": {"issue_active_pct": 70.8, "l1tex_pct": 82.5, "fma_pipe_pct": 55.1,
+                           "thread_inst_per_pair": 13.0, "shared_atomic_replay_pct": 48.6},
+               "backward": {"issue_active_pct": 76.2, "l1tex_pct": 53.1, "fma_pipe_pct": 64.0,
+                            "thread_inst_per_pair": 13.8},
                "source": "ncu, c2 geometry 256-layer slab: profiles/k_forward_tiled_strict_c2slab.md, "
                          "profiles/k_backward_tiled_strict_c2slab.md"},
-    "fast": {"forward": {"issue_active_pct": 65.7, "l1tex_pct": 96.5, "thread_inst_per_pair": 9.5},
-             "backward": {"issue_active_pct": 80.9, "thread_inst_per_pair": 10.7},
+    "fast": {"forward": {"issue_active_pct": 66.0, "l1tex_pct": 96.5, "thread_inst_per_pair": 9.5},
+             "backward": {"issue_active_pct": 81.1, "thread_inst_per_pair": 10.6},
              "source": "ncu, c2 geometry 256-layer slab: profiles/k_forward_tiled_fast_c2slab.md, "
                        "profiles/k_backward_tiled_fast_c2slab.md"},
 }
